@@ -63,7 +63,8 @@ template <typename T> struct ReinitWork {
     uint8_t *flags;
     Ptr6<T> dist;     // ENO3 only
     EdgeLists edges;  // ENO3 only (its setDistance)
-    Band band;
+    Band band;         // FP32 form
+    NodeList flagged;  // FP64 form: nodes with a distance flag
 };
 template <typename T> ReinitWork<T> carve_reinit(Bump &w, const Grid &g, bool own_dist)
 {
@@ -74,6 +75,7 @@ template <typename T> ReinitWork<T> carve_reinit(Bump &w, const Grid &g, bool ow
     for (int q = 0; q < 6; ++q) r.dist.p[q] = own_dist ? w.take<T>(g.num) : nullptr;
     r.edges = own_dist ? carve_edges(w, g) : EdgeLists{};
     r.band = carve_band<T>(w, g);
+    r.flagged = std::is_same<T, double>::value ? carve_list(w, g) : NodeList{nullptr, nullptr};
     return r;
 }
 
@@ -316,8 +318,6 @@ int check_ws(int op, const Grid &g, int elem, void *ws, size_t bytes)
         if (e_ != cudaSuccess) return e_;                                                                          \
     } while (0)
 
-template <typename T> constexpr bool fast_form() { return std::is_same<T, float>::value; }
-
 template <typename T> Ptr6<const T> cview(const Ptr6<T> &p)
 {
     Ptr6<const T> r;
@@ -345,29 +345,51 @@ inline cudaError_t tiled(int kind, bool eno3, Band &band, const float *s_in, con
     return launch_tiled_stage(kind, eno3, st, g, s);
 }
 
+// one stage of the plain FP64 form (stage input s_in, step-start field n_in, output out)
+inline cudaError_t reinit64(Kind64 kind, bool eno3, const ReinitWork<double> &w, const double *s_in, const double *n_in,
+                            double *out, Ptr6<const double> d, int stage, const Grid &g, cudaStream_t s)
+{
+    const Stage64 st{s_in, n_in, out, w.flags, d, Ptr6<const double>{}, Ptr3<const double>{}, nullptr, nullptr,
+                     w.flagged};
+    return launch_stage64(kind, eno3, st, stage, g, s);
+}
+inline cudaError_t extend64(Kind64 kind, bool eno3, const ExtendWork<double> &w, const double *s_in, const double *n_in,
+                            double *out, Ptr6<const double> d, int stage, const Grid &g, cudaStream_t s)
+{
+    const Stage64 st{s_in, n_in, out, w.flags, d, cview(w.cp), cview3(w.v), nullptr, nullptr, w.flagged};
+    return launch_stage64(kind, eno3, st, stage, g, s);
+}
+inline cudaError_t advect64(const double *s_in, const double *n_in, double *out, Ptr3<const double> v,
+                            const double *speed, const double *dt, int stage, const Grid &g, cudaStream_t s)
+{
+    const Stage64 st{s_in,  n_in, out, nullptr, Ptr6<const double>{}, Ptr6<const double>{}, v,
+                     speed, dt,   NodeList{nullptr, nullptr}};
+    return launch_stage64(K64_ADVECT, false, st, stage, g, s);
+}
+
+// one reinitialization stage of either form (none of the FP32 kernels' extension inputs)
+template <typename T>
+cudaError_t reinit_stage(bool eno3, ReinitWork<T> &w, const T *s_in, const T *n_in, T *out, Ptr6<const T> d, int stage,
+                         const Grid &g, cudaStream_t s)
+{
+    if constexpr (std::is_same<T, float>::value)
+        return tiled(0, eno3, w.band, s_in, n_in, out, w.flags, d, BandShadow{}, Ptr3<const float>{}, nullptr, nullptr,
+                     stage, g, s);
+    else
+        return reinit64(K64_REINIT, eno3, w, s_in, n_in, out, d, stage, g, s);
+}
+
 // `iters` TVD-RK3 reinitialization pseudo-steps of F in place (flags already classified)
 template <typename T>
 int reinit_loop(T *F, int iters, Ptr6<const T> d, ReinitWork<T> &w, const Grid &g, bool eno3, cudaStream_t s)
 {
-    const bool fast = fast_form<T>();
-    if constexpr (std::is_same<T, float>::value) {
-        if (int st = band_reset(w.band, s)) return st;
-        const BandShadow none{};
-        const Ptr3<const float> none3{};
-        for (int it = 0; it < iters; ++it) {
-            VSL_TRY(tiled(0, eno3, w.band, F, F, w.b, w.flags, d, none, none3, nullptr, nullptr, 0, g, s));
-            VSL_TRY(tiled(0, eno3, w.band, w.b, F, w.c, w.flags, d, none, none3, nullptr, nullptr, 1, g, s));
-            VSL_TRY(tiled(0, eno3, w.band, w.c, F, F, w.flags, d, none, none3, nullptr, nullptr, 2, g, s));
-        }
-        return VSL_OK;
-    } else {
-        for (int it = 0; it < iters; ++it) {
-            VSL_TRY(launch_reinit_stage<T>(F, F, w.b, w.flags, d, g, 0, eno3, fast, s));
-            VSL_TRY(launch_reinit_stage<T>(w.b, F, w.c, w.flags, d, g, 1, eno3, fast, s));
-            VSL_TRY(launch_reinit_stage<T>(w.c, F, F, w.flags, d, g, 2, eno3, fast, s));
-        }
-        return VSL_OK;
+    if (int st = band_reset(w.band, s)) return st;
+    for (int it = 0; it < iters; ++it) {
+        VSL_TRY(reinit_stage<T>(eno3, w, F, F, w.b, d, 0, g, s));
+        VSL_TRY(reinit_stage<T>(eno3, w, w.b, F, w.c, d, 1, g, s));
+        VSL_TRY(reinit_stage<T>(eno3, w, w.c, F, F, d, 2, g, s));
     }
+    return VSL_OK;
 }
 
 // one TVD-RK3 reinitialization pseudo-step of F in place, kernel launches only (the FP32
@@ -376,18 +398,10 @@ int reinit_loop(T *F, int iters, Ptr6<const T> d, ReinitWork<T> &w, const Grid &
 template <typename T>
 int reinit_pseudo_step(T *F, Ptr6<const T> d, ReinitWork<T> &w, const Grid &g, cudaStream_t s)
 {
-    if constexpr (std::is_same<T, float>::value) {
-        const BandShadow none{};
-        const Ptr3<const float> none3{};
-        w.band.seq = 0;
-        VSL_TRY(tiled(0, false, w.band, F, F, w.b, w.flags, d, none, none3, nullptr, nullptr, 0, g, s));
-        VSL_TRY(tiled(0, false, w.band, w.b, F, w.c, w.flags, d, none, none3, nullptr, nullptr, 1, g, s));
-        VSL_TRY(tiled(0, false, w.band, w.c, F, F, w.flags, d, none, none3, nullptr, nullptr, 2, g, s));
-    } else {
-        VSL_TRY(launch_reinit_stage<T>(F, F, w.b, w.flags, d, g, 0, false, false, s));
-        VSL_TRY(launch_reinit_stage<T>(w.b, F, w.c, w.flags, d, g, 1, false, false, s));
-        VSL_TRY(launch_reinit_stage<T>(w.c, F, F, w.flags, d, g, 2, false, false, s));
-    }
+    w.band.seq = 0;
+    VSL_TRY(reinit_stage<T>(false, w, F, F, w.b, d, 0, g, s));
+    VSL_TRY(reinit_stage<T>(false, w, w.b, F, w.c, d, 1, g, s));
+    VSL_TRY(reinit_stage<T>(false, w, w.c, F, F, d, 2, g, s));
     return VSL_OK;
 }
 
@@ -405,9 +419,8 @@ int extend_setup(const T *F, Ptr6<const T> d, const ExtendWork<T> &w, const Grid
 template <typename T>
 int extend_loop(T *C, int iters, Ptr6<const T> d, ExtendWork<T> &w, const Grid &g, bool eno3, cudaStream_t s)
 {
-    const bool fast = fast_form<T>();
-    Ptr3<const T> v = cview3(w.v);
     if constexpr (std::is_same<T, float>::value) {
+        const Ptr3<const T> v = cview3(w.v);
         // FP64 crossing values and the band's FP64 shadow of C (BandShadow)
         VSL_TRY(launch_crossing_mixed(C, d, w.cp64, w.flagged, g, eno3, s));
         VSL_TRY(launch_shadow_init(C, w.sh[0], w.flagged, s));
@@ -424,11 +437,10 @@ int extend_loop(T *C, int iters, Ptr6<const T> d, ExtendWork<T> &w, const Grid &
         return VSL_OK;
     } else {
         VSL_TRY(launch_crossing<T>(C, d, w.cp, w.flagged, g, eno3, s));
-        Ptr6<const T> cp = cview(w.cp);
         for (int it = 0; it < iters; ++it) {
-            VSL_TRY(launch_extend_stage<T>(C, C, w.b, w.flags, d, cp, v, g, 0, eno3, fast, s));
-            VSL_TRY(launch_extend_stage<T>(w.b, C, w.c, w.flags, d, cp, v, g, 1, eno3, fast, s));
-            VSL_TRY(launch_extend_stage<T>(w.c, C, C, w.flags, d, cp, v, g, 2, eno3, fast, s));
+            VSL_TRY(extend64(K64_EXTEND, eno3, w, C, C, w.b, d, 0, g, s));
+            VSL_TRY(extend64(K64_EXTEND, eno3, w, w.b, C, w.c, d, 1, g, s));
+            VSL_TRY(extend64(K64_EXTEND, eno3, w, w.c, C, C, d, 2, g, s));
         }
         return VSL_OK;
     }
@@ -438,7 +450,6 @@ template <typename T>
 int advect_loop(T *F, Ptr3<const T> v, const T *speed, const double *dt, int steps, ReinitWork<T> &w, const Grid &g,
                 cudaStream_t s)
 {
-    const bool fast = fast_form<T>();
     if constexpr (std::is_same<T, float>::value) {
         const Ptr6<const float> none6{};
         for (int it = 0; it < steps; ++it) {
@@ -449,9 +460,9 @@ int advect_loop(T *F, Ptr3<const T> v, const T *speed, const double *dt, int ste
         return VSL_OK;
     } else {
         for (int it = 0; it < steps; ++it) {
-            VSL_TRY(launch_advect_stage<T>(F, F, w.b, v, speed, dt, g, 0, fast, s));
-            VSL_TRY(launch_advect_stage<T>(w.b, F, w.c, v, speed, dt, g, 1, fast, s));
-            VSL_TRY(launch_advect_stage<T>(w.c, F, F, v, speed, dt, g, 2, fast, s));
+            VSL_TRY(advect64(F, F, w.b, v, speed, dt, 0, g, s));
+            VSL_TRY(advect64(w.b, F, w.c, v, speed, dt, 1, g, s));
+            VSL_TRY(advect64(w.c, F, F, v, speed, dt, 2, g, s));
         }
         return VSL_OK;
     }
@@ -495,7 +506,7 @@ int op_reinit_weno5(T *F, int iteration, const T *xpr, const T *xpl, const T *yp
     Bump b(ws);
     ReinitWork<T> w = carve_reinit<T>(b, g, false);
     Ptr6<const T> d = six(xpr, xpl, ypf, ypb, zpu, zpd);
-    VSL_TRY(launch_classify<T>(F, d, w.flags, NodeList{nullptr, nullptr}, g, s));
+    VSL_TRY(launch_classify<T>(F, d, w.flags, w.flagged, g, s));
     return reinit_loop<T>(F, iteration, d, w, g, false, s);
 }
 
@@ -513,7 +524,7 @@ int op_reinit_eno3(T *F, int iteration, int rows, int cols, int pges, double dx,
     ReinitWork<T> w = carve_reinit<T>(b, g, true);
     VSL_TRY(launch_set_distance<T>(F, w.dist, g, false, w.edges, s));
     Ptr6<const T> d = cview(w.dist);
-    VSL_TRY(launch_classify<T>(F, d, w.flags, NodeList{nullptr, nullptr}, g, s));
+    VSL_TRY(launch_classify<T>(F, d, w.flags, w.flagged, g, s));
     return reinit_loop<T>(F, iteration, d, w, g, true, s);
 }
 
@@ -573,20 +584,15 @@ int op_redistance(T *A, int iter1, int iter2, const T *F, int rows, int cols, in
     // reinitialization part: distances of A, mask A < 0 (ClosetPointSurfaceRedistance.m:15-25)
     VSL_TRY(launch_set_distance<T>(A, w.re.dist, g, !eno3, w.re.edges, s));
     Ptr6<const T> dA = cview(w.re.dist);
-    VSL_TRY(launch_classify<T>(A, dA, w.re.flags, NodeList{nullptr, nullptr}, g, s));
+    VSL_TRY(launch_classify<T>(A, dA, w.re.flags, w.re.flagged, g, s));
     // extension part: distances and upwind normals of F, floor 1e-14 (:37-74)
     VSL_TRY(launch_set_distance<T>(F, w.ext.dist, g, !eno3, w.ext.edges, s));
     Ptr6<const T> dF = cview(w.ext.dist);
     if (int st = extend_setup<T>(F, dF, w.ext, g, eno3, 1e-14, s)) return st;
-    const bool fast = fast_form<T>();
     if (int st = band_reset(w.re.band, s)) return st;
-    // one reinitialization stage of A's pseudo-time loop (tiled kernels for FP32)
-    auto re_stage = [&](const T *in, T *out, int stage) -> cudaError_t {
-        if constexpr (std::is_same<T, float>::value)
-            return tiled(0, eno3, w.re.band, in, A, out, w.re.flags, dA, BandShadow{}, Ptr3<const float>{},
-                         nullptr, nullptr, stage, g, s);
-        else
-            return launch_reinit_stage<T>(in, A, out, w.re.flags, dA, g, stage, eno3, fast, s);
+    // one reinitialization stage of A's pseudo-time loop
+    auto re_stage = [&](const T *in, T *out, int stage) {
+        return reinit_stage<T>(eno3, w.re, in, A, out, dA, stage, g, s);
     };
     // the reinit stages need their own temporaries: the extension uses w.ext.b/c
     T *t1 = w.re.b, *t2 = w.re.c;
@@ -727,7 +733,8 @@ int op_vesicle_step(T *F, T *xpr, T *xpl, T *ypf, T *ypb, T *zpu, T *zpd, int ex
     rw.c = w.ext.c;
     rw.flags = w.ext.flags;
     rw.band = w.ext.band;
-    VSL_TRY(launch_classify<T>(F, d, rw.flags, NodeList{nullptr, nullptr}, g, s));
+    if (std::is_same<T, double>::value) rw.flagged = w.ext.flagged;
+    VSL_TRY(launch_classify<T>(F, d, rw.flags, rw.flagged, g, s));
     return reinit_loop<T>(F, reinit_iters, d, rw, g, false, s);
 }
 
@@ -795,7 +802,7 @@ int record_reinit_tol(T *F, int max_iters, double tol, double band, Ptr6<const T
     VSL_TRY(cudaMemsetAsync(status, 0, 2 * sizeof(int), cap));
     VSL_TRY(cudaMemsetAsync(w.max_bits, 0, 2 * sizeof(unsigned long long), cap));
     if (int st = band_reset(w.re.band, cap)) return st;
-    VSL_TRY(launch_classify<T>(F, d, w.re.flags, NodeList{nullptr, nullptr}, g, cap));
+    VSL_TRY(launch_classify<T>(F, d, w.re.flags, w.re.flagged, g, cap));
     VSL_TRY(launch_reinit_residual<T>(F, w.re.flags, d, g, band, rs, cap));
     // the WHILE node after the prelude
     VSL_TRY(cudaStreamGetCaptureInfo(cap, &cs, nullptr, &graph, &deps, &edges, &ndeps));
@@ -1355,8 +1362,11 @@ int op_reinit_batch(const vsl_reinit_f32 *mem, int count, int iteration, cudaStr
 // ENORK2 (ENORK2Reinitialization.m:3-45, ENORK2Extend.m:9-81)
 // ---------------------------------------------------------------------------------------
 
-// the FP32 reinitialization workspace's band storage as a node list (the FP64 form has none)
-template <typename T> NodeList band_list(ReinitWork<T> &w) { return NodeList{w.band.q.queue, w.band.q.counter}; }
+// the reinitialization workspace's list of flagged nodes (FP32: its band storage)
+template <typename T> NodeList band_list(ReinitWork<T> &w)
+{
+    return std::is_same<T, float>::value ? NodeList{w.band.q.queue, w.band.q.counter} : w.flagged;
+}
 
 // one ENORK2 reinitialization stage; the FP32 form runs the tiled kernel on the uniform
 // nodes and the per-node code on the flagged list (from the classification) beside it
@@ -1369,7 +1379,7 @@ int enork2_reinit_stage(const T *in, const T *n_in, T *out, ReinitWork<T> &w, Pt
                       nullptr, stage, g, s, band_list(w)));
         return VSL_OK;
     } else {
-        VSL_TRY(launch_enork2_reinit_stage<T>(in, n_in, out, w.flags, d, g, stage, s));
+        VSL_TRY(reinit64(K64_ENO2R, false, w, in, n_in, out, d, stage, g, s));
         return VSL_OK;
     }
 }
@@ -1400,8 +1410,8 @@ int op_reinit_enork2(T *F, int iteration, int rows, int cols, int pges, double d
 template <typename T>
 int enork2_extend_loop(T *C, int iters, Ptr6<const T> d, ExtendWork<T> &w, const Grid &g, cudaStream_t s)
 {
-    const Ptr3<const T> v = cview3(w.v);
     if constexpr (std::is_same<T, float>::value) {
+        const Ptr3<const T> v = cview3(w.v);
         // tiled uniform nodes, the flagged list on the per-node code beside them with the FP64
         // crossing values and shadow of C
         VSL_TRY(launch_enork2_crossing_mixed(C, d, w.cp64, w.flagged, g, s));
@@ -1416,10 +1426,9 @@ int enork2_extend_loop(T *C, int iters, Ptr6<const T> d, ExtendWork<T> &w, const
         return VSL_OK;
     } else {
         VSL_TRY(launch_enork2_crossing<T>(C, d, w.cp, w.flagged, g, s));
-        const Ptr6<const T> cp = cview(w.cp);
         for (int it = 0; it < iters; ++it) {
-            VSL_TRY(launch_enork2_extend_stage<T>(C, C, w.b, w.flags, d, cp, v, g, 0, s));
-            VSL_TRY(launch_enork2_extend_stage<T>(w.b, C, C, w.flags, d, cp, v, g, 1, s));
+            VSL_TRY(extend64(K64_ENO2, false, w, C, C, w.b, d, 0, g, s));
+            VSL_TRY(extend64(K64_ENO2, false, w, w.b, C, C, d, 1, g, s));
         }
         return VSL_OK;
     }
@@ -1590,7 +1599,7 @@ int op_relax_step(T *F, T *xpr, T *xpl, T *ypf, T *ypb, T *zpu, T *zpd, double A
     VSL_TRY(launch_sum_partials(w.red.partials, nb, 1, ds3, ene, s));
     if (reinit_iters > 0) {
         const Ptr6<const T> d = six<T>(xpr, xpl, ypf, ypb, zpu, zpd);
-        VSL_TRY(launch_classify<T>(F, d, w.re.flags, NodeList{nullptr, nullptr}, g, s));
+        VSL_TRY(launch_classify<T>(F, d, w.re.flags, w.re.flagged, g, s));
         return reinit_loop<T>(F, reinit_iters, d, w.re, g, false, s);
     }
     return VSL_OK;
@@ -1630,8 +1639,8 @@ int advect_stages(const T *F, Ptr3<const T> v, const double *dt, ReinitWork<T> &
         VSL_TRY(tiled(2, false, w.band, F, F, w.b, nullptr, none6, BandShadow{}, v, nullptr, dt, 0, g, s));
         VSL_TRY(tiled(2, false, w.band, w.b, F, w.c, nullptr, none6, BandShadow{}, v, nullptr, dt, 1, g, s));
     } else {
-        VSL_TRY(launch_advect_stage<T>(F, F, w.b, v, nullptr, dt, g, 0, false, s));
-        VSL_TRY(launch_advect_stage<T>(w.b, F, w.c, v, nullptr, dt, g, 1, false, s));
+        VSL_TRY(advect64(F, F, w.b, v, nullptr, dt, 0, g, s));
+        VSL_TRY(advect64(w.b, F, w.c, v, nullptr, dt, 1, g, s));
     }
     return VSL_OK;
 }
@@ -1640,15 +1649,9 @@ int advect_stages(const T *F, Ptr3<const T> v, const double *dt, ReinitWork<T> &
 template <typename T>
 int reinit_stages(const T *F, Ptr6<const T> d, ReinitWork<T> &w, const Grid &g, cudaStream_t s)
 {
-    if constexpr (std::is_same<T, float>::value) {
-        if (int st = band_reset(w.band, s)) return st;
-        const Ptr3<const float> none3{};
-        VSL_TRY(tiled(0, false, w.band, F, F, w.b, w.flags, d, BandShadow{}, none3, nullptr, nullptr, 0, g, s));
-        VSL_TRY(tiled(0, false, w.band, w.b, F, w.c, w.flags, d, BandShadow{}, none3, nullptr, nullptr, 1, g, s));
-    } else {
-        VSL_TRY(launch_reinit_stage<T>(F, F, w.b, w.flags, d, g, 0, false, false, s));
-        VSL_TRY(launch_reinit_stage<T>(w.b, F, w.c, w.flags, d, g, 1, false, false, s));
-    }
+    if (int st = band_reset(w.band, s)) return st;
+    VSL_TRY(reinit_stage<T>(false, w, F, F, w.b, d, 0, g, s));
+    VSL_TRY(reinit_stage<T>(false, w, w.b, F, w.c, d, 1, g, s));
     return VSL_OK;
 }
 
@@ -1691,7 +1694,7 @@ int op_reinit_adjoint(const T *F0, int iteration, T *lam, T *tape, int rows, int
     // classification, then the pseudo-step inputs phi^0 .. phi^{K-1} into the tape
     VSL_TRY(launch_set_distance<T>(F0, re.dist, g, true, re.edges, s));
     const Ptr6<const T> d = cview(re.dist);
-    VSL_TRY(launch_classify<T>(F0, d, re.flags, NodeList{nullptr, nullptr}, g, s));
+    VSL_TRY(launch_classify<T>(F0, d, re.flags, re.flagged, g, s));
     const size_t field = sizeof(T) * (size_t)g.num;
     VSL_TRY(cudaMemcpyAsync(tape, F0, field, cudaMemcpyDeviceToDevice, s));
     for (int k = 1; k < iteration; ++k) {

@@ -1,8 +1,10 @@
-// vsl_fused.cuh -- fused TVD-RK3 stage kernels of the method-level operations, included
-// by vsl_fused_f64.cu (plain form, compiled without multiply-add contraction so that the
-// FP64 arithmetic rounds like the reference's) and vsl_fused_f32.cu (mixed form).
+// vsl_fused.cuh -- per-node code of the fused TVD-RK3 stages of the method-level operations
+// and their set-up kernels, included by vsl_fused_f64.cu (plain form, compiled without
+// multiply-add contraction so that the FP64 arithmetic rounds like the reference's; stage
+// kernels in vsl_stage64.cuh) and vsl_fused_f32.cu (mixed form; stage kernels in
+// vsl_tiled.cuh).
 //
-// One launch evaluates one Runge-Kutta stage of a whole pseudo-step AND its Shu-Osher
+// One stage evaluates one Runge-Kutta stage of a whole pseudo-step AND its Shu-Osher
 // combination, writing the next stage field directly:
 //   stage 0: out = phi_s - step(phi_s)
 //   stage 1: out = 3/4 phi_n + 1/4 (phi_s - step(phi_s))
@@ -305,16 +307,6 @@ __device__ __forceinline__ void reinit_node(const T *__restrict__ phi_s, const T
     out[c] = rk3_combine(stage, pn, ps - step);
 }
 
-template <typename T, bool ENO3, bool FAST>
-__global__ void __launch_bounds__(BX *BY) k_reinit_stage(const T *__restrict__ phi_s, const T *__restrict__ phi_n,
-                                                           T *__restrict__ out, const uint8_t *__restrict__ flags,
-                                                           Ptr6<const T> d, Grid g, int stage)
-{
-    int i, j, k;
-    if (!fused_node(g, i, j, k)) return;
-    reinit_node<T, ENO3, FAST>(phi_s, phi_n, out, flags, d, g, stage, i, j, k);
-}
-
 // ---------------------------------------------------------------------------------------
 // reinitialization residual
 // ---------------------------------------------------------------------------------------
@@ -435,16 +427,6 @@ __device__ __forceinline__ void extension_velocity_node(const T *__restrict__ ph
     for (int ax = 0; ax < 3; ++ax) v.p[ax][c] = s * (n[ax] / grad);
 }
 
-template <typename T, bool ENO3>
-__global__ void __launch_bounds__(BX *BY) k_extension_velocity(const T *__restrict__ phi,
-                                                                 const uint8_t *__restrict__ flags, Ptr6<const T> d,
-                                                                 Ptr3<T> v, Grid g, T floor)
-{
-    int i, j, k;
-    if (!fused_node(g, i, j, k)) return;
-    extension_velocity_node<T, ENO3>(phi, flags, d, v, g, floor, i, j, k);
-}
-
 // The mixed form splits the extension velocity: nodes without a distance flag take the
 // uniform path on 2.5D tiles (stage kind SK_VELOCITY), where only the side each axis keeps
 // (n = D+ where |p4| < |p2|, else D-) is reconstructed, x and y as the two lanes of one
@@ -543,29 +525,17 @@ __device__ __forceinline__ void extend_node(const T *__restrict__ c_s, const T *
     out[c] = rk3_combine(stage, pn, cs - step);
 }
 
-template <typename T, bool ENO3, bool FAST>
-__global__ void __launch_bounds__(BX *BY) k_extend_stage(const T *__restrict__ c_s, const T *__restrict__ c_n,
-                                                           T *__restrict__ out, const uint8_t *__restrict__ flags,
-                                                           Ptr6<const T> d, Ptr6<const T> cp, Ptr3<const T> v, Grid g,
-                                                           int stage)
-{
-    int i, j, k;
-    if (!fused_node(g, i, j, k)) return;
-    extend_node<T, ENO3, FAST>(c_s, c_n, out, flags, d, cp, v, g, stage, i, j, k);
-}
-
 // ---------------------------------------------------------------------------------------
 // WENO5 advection stage: step = dt * (upwind v.grad phi) (advection_step.cu:30-56).
 // With `speed` non-null the velocity is speed * (v0, v1, v2) (normal speed times normal).
 // ---------------------------------------------------------------------------------------
+// one node of an advection stage, all reads from global memory (clamped)
 template <typename T, bool FAST>
-__global__ void __launch_bounds__(BX *BY) k_advect_stage(const T *__restrict__ phi_s, const T *__restrict__ phi_n,
-                                                           T *__restrict__ out, Ptr3<const T> v,
-                                                           const T *__restrict__ speed, const double *__restrict__ dt,
-                                                           Grid g, int stage)
+__device__ __forceinline__ void advect_node(const T *__restrict__ phi_s, const T *__restrict__ phi_n,
+                                            T *__restrict__ out, const Ptr3<const T> &v, const T *__restrict__ speed,
+                                            const double *__restrict__ dt, const Grid &g, int stage, int i, int j,
+                                            int k)
 {
-    int i, j, k;
-    if (!fused_node(g, i, j, k)) return;
     const long long c = node_index(g, i, j, k);
     T df[3], db[3];
 #pragma unroll
@@ -648,17 +618,6 @@ __device__ __forceinline__ void enork2_reinit_node(const T *__restrict__ phi_s, 
     out[c] = rk2_combine(stage, pn, __ldg(phi_s + c), step);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(BX *BY) k_enork2_reinit_stage(const T *__restrict__ phi_s,
-                                                                  const T *__restrict__ phi_n, T *__restrict__ out,
-                                                                  const uint8_t *__restrict__ flags, Ptr6<const T> d,
-                                                                  Grid g, int stage)
-{
-    int i, j, k;
-    if (!fused_node(g, i, j, k)) return;
-    enork2_reinit_node<T>(phi_s, phi_n, out, flags, d, g, stage, i, j, k);
-}
-
 // v = sign(F) * n / max(|n|, floor) with the ENO upwind normal (enork2_extend.cu:103-141,
 // ENORK2Extend.m:26-42)
 template <typename T>
@@ -729,17 +688,6 @@ __device__ __forceinline__ void enork2_extend_node(const T *__restrict__ c_s, co
     out[c] = rk2_combine(stage, pn, __ldg(c_s + c), step);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(BX *BY) k_enork2_extend_stage(const T *__restrict__ c_s, const T *__restrict__ c_n,
-                                                                  T *__restrict__ out, const uint8_t *__restrict__ flags,
-                                                                  Ptr6<const T> d, Ptr6<const T> cp, Ptr3<const T> v,
-                                                                  Grid g, int stage)
-{
-    int i, j, k;
-    if (!fused_node(g, i, j, k)) return;
-    enork2_extend_node<T>(c_s, c_n, out, flags, d, cp, v, g, stage, i, j, k);
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------------------
@@ -795,47 +743,6 @@ cudaError_t launch_classify(const T *phi0, Ptr6<const T> dist, uint8_t *flags, N
 }
 
 template <typename T>
-cudaError_t launch_reinit_stage(const T *phi_s, const T *phi_n, T *out, const uint8_t *flags, Ptr6<const T> dist,
-                                const Grid &g, int stage, bool eno3, bool fast, cudaStream_t s)
-{
-    dim3 gr = node_grid(g), bl(BX, BY);
-    if (eno3) {
-        if (fast)
-            k_reinit_stage<T, true, true><<<gr, bl, 0, s>>>(phi_s, phi_n, out, flags, dist, g, stage);
-        else
-            k_reinit_stage<T, true, false><<<gr, bl, 0, s>>>(phi_s, phi_n, out, flags, dist, g, stage);
-    } else {
-        if (fast)
-            k_reinit_stage<T, false, true><<<gr, bl, 0, s>>>(phi_s, phi_n, out, flags, dist, g, stage);
-        else
-            k_reinit_stage<T, false, false><<<gr, bl, 0, s>>>(phi_s, phi_n, out, flags, dist, g, stage);
-    }
-    return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch_extension_velocity(const T *phi, const uint8_t *flags, Ptr6<const T> dist, Ptr3<T> v, const Grid &g,
-                                      bool eno3, double floor, NodeList flagged, cudaStream_t s)
-{
-    if constexpr (std::is_same<T, float>::value) {
-        if (flagged.idx) {
-            cudaError_t err = launch_velocity_tiled(phi, flags, v, g, (float)floor, s);
-            if (err != cudaSuccess) return err;
-            if (eno3)
-                k_velocity_list<true><<<list_blocks(), 128, 0, s>>>(phi, flags, dist, v, flagged, g, (float)floor);
-            else
-                k_velocity_list<false><<<list_blocks(), 128, 0, s>>>(phi, flags, dist, v, flagged, g, (float)floor);
-            return cudaGetLastError();
-        }
-    }
-    if (eno3)
-        k_extension_velocity<T, true><<<node_grid(g), dim3(BX, BY), 0, s>>>(phi, flags, dist, v, g, (T)floor);
-    else
-        k_extension_velocity<T, false><<<node_grid(g), dim3(BX, BY), 0, s>>>(phi, flags, dist, v, g, (T)floor);
-    return cudaGetLastError();
-}
-
-template <typename T>
 cudaError_t launch_crossing(const T *c, Ptr6<const T> dist, Ptr6<T> cp, NodeList list, const Grid &g, bool cubic,
                             cudaStream_t s)
 {
@@ -847,51 +754,12 @@ cudaError_t launch_crossing(const T *c, Ptr6<const T> dist, Ptr6<T> cp, NodeList
 }
 
 template <typename T>
-cudaError_t launch_extend_stage(const T *c_s, const T *c_n, T *out, const uint8_t *flags, Ptr6<const T> dist,
-                                Ptr6<const T> cp, Ptr3<const T> v, const Grid &g, int stage, bool eno3, bool fast,
-                                cudaStream_t s)
-{
-    dim3 gr = node_grid(g), bl(BX, BY);
-    if (eno3) {
-        if (fast)
-            k_extend_stage<T, true, true><<<gr, bl, 0, s>>>(c_s, c_n, out, flags, dist, cp, v, g, stage);
-        else
-            k_extend_stage<T, true, false><<<gr, bl, 0, s>>>(c_s, c_n, out, flags, dist, cp, v, g, stage);
-    } else {
-        if (fast)
-            k_extend_stage<T, false, true><<<gr, bl, 0, s>>>(c_s, c_n, out, flags, dist, cp, v, g, stage);
-        else
-            k_extend_stage<T, false, false><<<gr, bl, 0, s>>>(c_s, c_n, out, flags, dist, cp, v, g, stage);
-    }
-    return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch_advect_stage(const T *phi_s, const T *phi_n, T *out, Ptr3<const T> v, const T *speed,
-                                const double *dt, const Grid &g, int stage, bool fast, cudaStream_t s)
-{
-    if (fast)
-        k_advect_stage<T, true><<<node_grid(g), dim3(BX, BY), 0, s>>>(phi_s, phi_n, out, v, speed, dt, g, stage);
-    else
-        k_advect_stage<T, false><<<node_grid(g), dim3(BX, BY), 0, s>>>(phi_s, phi_n, out, v, speed, dt, g, stage);
-    return cudaGetLastError();
-}
-
-template <typename T>
 cudaError_t launch_set_distance_eno2(const T *phi, Ptr6<T> dist, const Grid &g, EdgeLists e, cudaStream_t s)
 {
     cudaError_t err = cudaMemsetAsync(e.count, 0, 3 * sizeof(unsigned), s);
     if (err != cudaSuccess) return err;
     k_dist_scan<T><<<node_grid(g), dim3(BX, BY), 0, s>>>(phi, dist, e, g);
     k_dist_roots_eno2<T><<<list_blocks() * 4, 128, 0, s>>>(phi, dist, e, g);
-    return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch_enork2_reinit_stage(const T *phi_s, const T *phi_n, T *out, const uint8_t *flags,
-                                       Ptr6<const T> dist, const Grid &g, int stage, cudaStream_t s)
-{
-    k_enork2_reinit_stage<T><<<node_grid(g), dim3(BX, BY), 0, s>>>(phi_s, phi_n, out, flags, dist, g, stage);
     return cudaGetLastError();
 }
 
@@ -912,14 +780,6 @@ cudaError_t launch_enork2_crossing(const T *c, Ptr6<const T> dist, Ptr6<T> cp, N
 }
 
 template <typename T>
-cudaError_t launch_enork2_extend_stage(const T *c_s, const T *c_n, T *out, const uint8_t *flags, Ptr6<const T> dist,
-                                       Ptr6<const T> cp, Ptr3<const T> v, const Grid &g, int stage, cudaStream_t s)
-{
-    k_enork2_extend_stage<T><<<node_grid(g), dim3(BX, BY), 0, s>>>(c_s, c_n, out, flags, dist, cp, v, g, stage);
-    return cudaGetLastError();
-}
-
-template <typename T>
 cudaError_t launch_reinit_residual(const T *phi, const uint8_t *flags, Ptr6<const T> dist, const Grid &g, double band,
                                    const ResidualState &st, cudaStream_t s)
 {
@@ -931,27 +791,10 @@ cudaError_t launch_reinit_residual(const T *phi, const uint8_t *flags, Ptr6<cons
     template cudaError_t launch_set_distance<T>(const T *, Ptr6<T>, const Grid &, bool, EdgeLists, cudaStream_t);   \
     template cudaError_t launch_classify<T>(const T *, Ptr6<const T>, uint8_t *, NodeList, const Grid &,            \
                                             cudaStream_t);                                                          \
-    template cudaError_t launch_reinit_stage<T>(const T *, const T *, T *, const uint8_t *, Ptr6<const T>,          \
-                                                const Grid &, int, bool, bool, cudaStream_t);                       \
-    template cudaError_t launch_extension_velocity<T>(const T *, const uint8_t *, Ptr6<const T>, Ptr3<T>,           \
-                                                      const Grid &, bool, double, NodeList, cudaStream_t);          \
     template cudaError_t launch_reinit_residual<T>(const T *, const uint8_t *, Ptr6<const T>, const Grid &, double, \
                                                    const ResidualState &, cudaStream_t);                           \
-    template cudaError_t launch_crossing<T>(const T *, Ptr6<const T>, Ptr6<T>, NodeList, const Grid &, bool,        \
-                                            cudaStream_t);                                                          \
-    template cudaError_t launch_extend_stage<T>(const T *, const T *, T *, const uint8_t *, Ptr6<const T>,          \
-                                                Ptr6<const T>, Ptr3<const T>, const Grid &, int, bool, bool,        \
-                                                cudaStream_t);                                                      \
-    template cudaError_t launch_advect_stage<T>(const T *, const T *, T *, Ptr3<const T>, const T *,                \
-                                                const double *, const Grid &, int, bool, cudaStream_t);             \
     template cudaError_t launch_set_distance_eno2<T>(const T *, Ptr6<T>, const Grid &, EdgeLists, cudaStream_t);    \
-    template cudaError_t launch_enork2_reinit_stage<T>(const T *, const T *, T *, const uint8_t *, Ptr6<const T>,   \
-                                                       const Grid &, int, cudaStream_t);                            \
     template cudaError_t launch_enork2_velocity<T>(const T *, Ptr6<const T>, Ptr3<T>, const Grid &, double,         \
-                                                   cudaStream_t);                                                   \
-    template cudaError_t launch_enork2_crossing<T>(const T *, Ptr6<const T>, Ptr6<T>, NodeList, const Grid &,       \
-                                                   cudaStream_t);                                                   \
-    template cudaError_t launch_enork2_extend_stage<T>(const T *, const T *, T *, const uint8_t *, Ptr6<const T>,   \
-                                                       Ptr6<const T>, Ptr3<const T>, const Grid &, int, cudaStream_t);
+                                                   cudaStream_t);
 
 }  // namespace vsl

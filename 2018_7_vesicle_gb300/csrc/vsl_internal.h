@@ -72,11 +72,8 @@ cudaError_t launch_set_distance(const T *phi, Ptr6<T> dist, const Grid &g, bool 
 template <typename T>
 cudaError_t launch_classify(const T *phi0, Ptr6<const T> dist, uint8_t *flags, NodeList list, const Grid &g,
                             cudaStream_t s);
-template <typename T>
-cudaError_t launch_reinit_stage(const T *phi_s, const T *phi_n, T *out, const uint8_t *flags, Ptr6<const T> dist,
-                                const Grid &g, int stage, bool eno3, bool fast, cudaStream_t s);
 // flags: the classification bytes of phi with these distances (launch_classify); flagged:
-// its list of flagged nodes (the FP32 form then runs the uniform nodes and the list apart)
+// its list of flagged nodes (the uniform nodes and the list run apart)
 template <typename T>
 cudaError_t launch_extension_velocity(const T *phi, const uint8_t *flags, Ptr6<const T> dist, Ptr3<T> v, const Grid &g,
                                       bool eno3, double floor, NodeList flagged, cudaStream_t s);
@@ -84,14 +81,6 @@ cudaError_t launch_extension_velocity(const T *phi, const uint8_t *flags, Ptr6<c
 template <typename T>
 cudaError_t launch_crossing(const T *c, Ptr6<const T> dist, Ptr6<T> cp, NodeList list, const Grid &g, bool cubic,
                             cudaStream_t s);
-template <typename T>
-cudaError_t launch_extend_stage(const T *c_s, const T *c_n, T *out, const uint8_t *flags, Ptr6<const T> dist,
-                                Ptr6<const T> cp, Ptr3<const T> v, const Grid &g, int stage, bool eno3, bool fast,
-                                cudaStream_t s);
-template <typename T>
-cudaError_t launch_advect_stage(const T *phi_s, const T *phi_n, T *out, Ptr3<const T> v, const T *speed,
-                                const double *dt, const Grid &g, int stage, bool fast, cudaStream_t s);
-
 // Reinitialization residual (no counterpart in the reference, whose loops run a fixed
 // count): the FP64 maximum over the band |phi| < band of | |grad phi|_G - 1 |, the Godunov
 // norm the stage takes, at the non-fixed nodes.  The last block to finish records it and
@@ -115,22 +104,30 @@ cudaError_t launch_reinit_residual(const T *phi, const uint8_t *flags, Ptr6<cons
 // iteration, so that only a completed residual evaluation can continue the loop)
 cudaError_t launch_condition_reset(cudaGraphConditionalHandle handle, cudaStream_t s);
 
-// ENORK2 (second-order ENO, Heun RK2 stages 0 and 1): quadratic-ENO distances, the
-// reinitialization and extension stages, the extension velocity and crossing values
+// ENORK2 (second-order ENO): quadratic-ENO distances, the extension velocity and crossing
+// values
 template <typename T>
 cudaError_t launch_set_distance_eno2(const T *phi, Ptr6<T> dist, const Grid &g, EdgeLists e, cudaStream_t s);
-template <typename T>
-cudaError_t launch_enork2_reinit_stage(const T *phi_s, const T *phi_n, T *out, const uint8_t *flags,
-                                       Ptr6<const T> dist, const Grid &g, int stage, cudaStream_t s);
 template <typename T>
 cudaError_t launch_enork2_velocity(const T *phi, Ptr6<const T> dist, Ptr3<T> v, const Grid &g, double floor,
                                    cudaStream_t s);
 template <typename T>
 cudaError_t launch_enork2_crossing(const T *c, Ptr6<const T> dist, Ptr6<T> cp, NodeList list, const Grid &g,
                                    cudaStream_t s);
-template <typename T>
-cudaError_t launch_enork2_extend_stage(const T *c_s, const T *c_n, T *out, const uint8_t *flags, Ptr6<const T> dist,
-                                       Ptr6<const T> cp, Ptr3<const T> v, const Grid &g, int stage, cudaStream_t s);
+// ---- stage kernels of the plain FP64 form (vsl_stage64.cuh, built into vsl_fused_f64.cu) --
+// REINIT, EXTEND: WENO5 with the nonuniform WENO (or, with eno3, cubic ENO) interface stencils;
+// ENO2, ENO2R: the ENORK2 extension and reinitialization; VELOCITY: the extension velocity
+enum Kind64 { K64_REINIT, K64_EXTEND, K64_ADVECT, K64_VELOCITY, K64_ENO2, K64_ENO2R };
+struct Stage64 {
+    const double *phi_s, *phi_n;
+    double *out;
+    const uint8_t *flags;
+    Ptr6<const double> d, cp;
+    Ptr3<const double> v;
+    const double *speed, *dt;
+    NodeList flagged;  // the classification's list (all kinds but ADVECT)
+};
+cudaError_t launch_stage64(Kind64 kind, bool eno3, const Stage64 &st, int stage, const Grid &g, cudaStream_t s);
 
 // ---- the relaxation step (vsl_relax.cuh, vsl_spectral.cu), T in {float, double} ------
 template <typename T> cudaError_t launch_laplacian(const T *f, T *out, const Grid &g, cudaStream_t s);

@@ -1,0 +1,411 @@
+// vsl_stage64.cuh -- stage kernels of the plain FP64 form on cheaper arithmetic with the
+// same results, bit for bit, as the per-node functions of vsl_fused.cuh.
+//
+// What bounds these kernels is the FP64 pipe: two lanes per SM and clock on GB300, 1/64 of
+// the FP32 rate, so a warp's FP64 instruction occupies it for 16 cycles and everything else
+// (loads, integer work, selects) is free beside it.  A node of the per-node form costs about
+// 1100 FP64 instructions per stage: 24 quotients per axis as general divisions, and both
+// one-sided derivatives of every axis.  Here:
+//   * quotients by the grid spacing take its correctly rounded reciprocal (formed on the
+//     host) and the multiply / remainder / correction sequence of Markstein (IBM J. Res.
+//     Dev. 34, 1990): three instructions, the correctly rounded quotient;
+//   * the WENO weights' quotients share one reciprocal per divisor, from the documented PTX
+//     approximation rcp.approx.ftz.f64 and one third-order Newton step (error 1 - b y cubed);
+//   * multiplications by powers of two ride in an FMA, which rounds the same;
+//   * transport evaluates only the upwind side of an axis (the other is multiplied by zero),
+//     and the Godunov norm only the sides whose three candidate values do not all have the
+//     sign that the maximum with zero discards (the weights are positive, so the
+//     reconstruction lies between the candidates);
+//   * nodes with an interface distance ("flagged", the classification's list) are updated by
+//     band blocks at the front of the same launch with the general per-node code, so that no
+//     warp of the others runs the nonuniform stencils for a few of its lanes.
+// About 310 / 350 FP64 instructions per node and stage (transport / norm).
+//
+// The sequences above need operands away from overflow and underflow.  A node whose stencil
+// holds a value that is neither zero nor of magnitude 2^-400 .. 2^100 (infinities and NaN
+// among them), and a reinitialization node that has a sign change but no distance flag, takes
+// the general code.  Spacings outside 2^-60 .. 2^60 send every node there.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+
+#include "vsl_fused.cuh"
+
+namespace vsl {
+namespace {
+
+// ---------------------------------------------------------------------------------------
+// quotients
+// ---------------------------------------------------------------------------------------
+
+// a / d for the divisor d whose reciprocal r is 1 / d to within an ulp
+__device__ __forceinline__ double quotient(double a, double d, double r)
+{
+    const double q = __dmul_rn(a, r);
+    return __fma_rn(__fma_rn(-d, q, a), r, q);
+}
+
+// 1 / d to within an ulp for a normal d whose reciprocal is normal
+__device__ __forceinline__ double reciprocal(double d)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = __fma_rn(-d, y, 1.0);  // at most about 2^-19
+    return __fma_rn(y, __fma_rn(e, e, e), y);
+}
+
+// magnitude bits of the high word
+__device__ __forceinline__ int mag_hi(double x) { return __double2hiint(x) & 0x7fffffff; }
+// zero, or of magnitude 2^-400 .. 2^100
+__device__ __forceinline__ bool ordinary(double x)
+{
+    const unsigned m = (unsigned)mag_hi(x);
+    return m - (unsigned)((1023 - 400) << 20) < (unsigned)(500 << 20) || (m | (unsigned)__double2loint(x)) == 0u;
+}
+__device__ __forceinline__ bool sign_bit(double x) { return __double2hiint(x) < 0; }
+__device__ __forceinline__ double flip(double x, bool neg)
+{
+    return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
+
+// ---------------------------------------------------------------------------------------
+// WENO5 (weno5_plain, the same roundings)
+// ---------------------------------------------------------------------------------------
+
+// the three candidate values of the window v1..v5
+__device__ __forceinline__ void candidates64(double v1, double v2, double v3, double v4, double v5, double q[3])
+{
+    q[0] = 1. / 3. * v1 - 7. / 6. * v2 + 11. / 6. * v3;
+    q[1] = 5. / 6. * v3 - 1. / 6. * v2 + 1. / 3. * v4;
+    q[2] = 1. / 3. * v3 + 5. / 6. * v4 - 1. / 6. * v5;
+}
+
+// the weighted value of the candidates q of the window v1..v5
+__device__ __forceinline__ double weighted64(double v1, double v2, double v3, double v4, double v5, const double q[3])
+{
+    const double t3 = 3.0 * v3;
+    const double s1 = __fma_rn(0.25, sqr(__fma_rn(-4.0, v2, v1) + t3), 13. / 12. * sqr(__fma_rn(-2.0, v2, v1) + v3));
+    const double s2 = __fma_rn(0.25, sqr(v2 - v4), 13. / 12. * sqr(__fma_rn(-2.0, v3, v2) + v4));
+    const double s3 = __fma_rn(0.25, sqr(__fma_rn(-4.0, v4, t3) + v5), 13. / 12. * sqr(__fma_rn(-2.0, v4, v3) + v5));
+    const double b1 = sqr(s1 + 1e-6), b2 = sqr(s2 + 1e-6), b3 = sqr(s3 + 1e-6);
+    const double a1 = quotient(0.1, b1, reciprocal(b1));
+    const double a2 = quotient(0.6, b2, reciprocal(b2));
+    const double a3 = quotient(0.3, b3, reciprocal(b3));
+    const double tot = a1 + a2 + a3, r = reciprocal(tot);
+    return quotient(a1, tot, r) * q[0] + quotient(a2, tot, r) * q[1] + quotient(a3, tot, r) * q[2];
+}
+
+// D- at t[3] of the line t (six points, t[3] the node); the line mirrored about the node
+// gives -D+
+__device__ __forceinline__ double upwind64(const double t[6], double h, double rh)
+{
+    double v[5], q[3];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) v[m] = quotient(t[m + 1] - t[m], h, rh);
+    candidates64(v[0], v[1], v[2], v[3], v[4], q);
+    return weighted64(v[0], v[1], v[2], v[3], v[4], q);
+}
+
+// max(0, D-, -D+) of the line p, with both derivatives negated where neg (godunov_norm's
+// term before the square)
+__device__ __forceinline__ double godunov_side64(const double p[7], bool neg, double h, double rh)
+{
+    double u[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) u[m] = quotient(p[m + 1] - p[m], h, rh);
+    double qb[3], qf[3];
+    {
+        const double s1 = 1. / 6. * u[1], s4 = 1. / 6. * u[4], h2 = 1. / 3. * u[2], h3 = 1. / 3. * u[3];
+        const double f2 = 5. / 6. * u[2], f3 = 5. / 6. * u[3];
+        qb[0] = 1. / 3. * u[0] - 7. / 6. * u[1] + 11. / 6. * u[2];
+        qb[1] = f2 - s1 + h3;
+        qb[2] = h2 + f3 - s4;
+        qf[0] = 1. / 3. * u[5] - 7. / 6. * u[4] + 11. / 6. * u[3];
+        qf[1] = f3 - s4 + h2;
+        qf[2] = h3 + f2 - s1;
+    }
+    // D- counts where positive (neg: negative), D+ where negative (neg: positive)
+    const bool b = neg ? sign_bit(qb[0]) || sign_bit(qb[1]) || sign_bit(qb[2])
+                       : !(sign_bit(qb[0]) && sign_bit(qb[1]) && sign_bit(qb[2]));
+    const bool f = neg ? !(sign_bit(qf[0]) && sign_bit(qf[1]) && sign_bit(qf[2]))
+                       : sign_bit(qf[0]) || sign_bit(qf[1]) || sign_bit(qf[2]);
+    const double q[3] = {b ? qb[0] : qf[0], b ? qb[1] : qf[1], b ? qb[2] : qf[2]};
+    double e = weighted64(b ? u[0] : u[5], b ? u[1] : u[4], b ? u[2] : u[3], b ? u[3] : u[2], b ? u[4] : u[1], q);
+    e = flip(e, neg == b);
+    e = (b || f) && !sign_bit(e) ? e : 0.0;
+    if (b && f) {
+        const double g = flip(weighted64(u[5], u[4], u[3], u[2], u[1], qf), !neg);
+        e = g > e ? g : e;
+    }
+    return e;
+}
+
+// ---------------------------------------------------------------------------------------
+// quadratic ENO (eno2_pair with r1 = l1 = h, the same roundings)
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ double minmod64(double x, double y)
+{
+    const long long a = __double_as_longlong(x), b = __double_as_longlong(y), m = 0x7fffffffffffffffLL;
+    const double s = (a & m) < (b & m) ? x : y;
+    return (a ^ b) < 0 ? 0.0 : s;  // of opposite sign (or one a zero)
+}
+
+// Backward quadratic-ENO derivative at t3 of the points t1, t2, t3 (t3 the node); the mirrored
+// points give the forward one negated.  c: the second difference at the node (the same sum for
+// both sides), h2 = h * h, rh2 its reciprocal.
+__device__ __forceinline__ double eno2_back64(double t1, double t2, double t3, double c, double h, double rh,
+                                              double h2, double rh2)
+{
+    const double l = __fma_rn(-2.0, t2, t3) + t1;
+    return quotient(t3 - t2, h, rh) + (0.5 * h) * quotient(minmod64(c, l), h2, rh2);
+}
+
+// ---------------------------------------------------------------------------------------
+// the stage kernel
+// ---------------------------------------------------------------------------------------
+__host__ __device__ constexpr bool band_kind64(int kind) { return kind != K64_ADVECT; }
+__host__ __device__ constexpr bool transport_kind64(int kind)
+{
+    return kind == K64_EXTEND || kind == K64_ADVECT || kind == K64_ENO2;
+}
+
+struct Args64 {
+    Stage64 st;
+    Ptr3<double> w;  // VELOCITY: the velocity written
+    int band_blocks;
+    Grid g;
+    double h[3], rh[3], h2[3], rh2[3];
+    double dt_uniform;  // 0.3 * min spacing: the pseudo time step of a node without a flag
+    double floor;       // VELOCITY: the floor of |grad phi|
+    bool ordinary;      // the spacings are within the range of the short sequences
+};
+
+// One node by the general code (vsl_fused.cuh): band nodes, and the nodes whose stencil the
+// short sequences do not take.
+template <int KIND, int STAGE, bool ENO3> __device__ __forceinline__ void general_node64(const Args64 &a, long long c)
+{
+    const Grid &g = a.g;
+    int i, j, k;
+    node_of(g, c, i, j, k);
+    if constexpr (KIND == K64_REINIT) {
+        reinit_node<double, ENO3, false>(a.st.phi_s, a.st.phi_n, a.st.out, a.st.flags, a.st.d, g, STAGE, i, j, k);
+    } else if constexpr (KIND == K64_EXTEND) {
+        extend_node<double, ENO3, false>(a.st.phi_s, a.st.phi_n, a.st.out, a.st.flags, a.st.d, a.st.cp, a.st.v, g, STAGE, i, j, k);
+    } else if constexpr (KIND == K64_ADVECT) {
+        advect_node<double, false>(a.st.phi_s, a.st.phi_n, a.st.out, a.st.v, a.st.speed, a.st.dt, g, STAGE, i, j, k);
+    } else if constexpr (KIND == K64_VELOCITY) {
+        Ptr3<double> w = a.w;
+        extension_velocity_node<double, ENO3>(a.st.phi_s, a.st.flags, a.st.d, w, g, a.floor, i, j, k);
+    } else if constexpr (KIND == K64_ENO2) {
+        enork2_extend_node<double>(a.st.phi_s, a.st.phi_n, a.st.out, a.st.flags, a.st.d, a.st.cp, a.st.v, g, STAGE, i, j, k);
+    } else {
+        enork2_reinit_node<double>(a.st.phi_s, a.st.phi_n, a.st.out, a.st.flags, a.st.d, g, STAGE, i, j, k);
+    }
+}
+template <int KIND, int STAGE, bool ENO3> __device__ __noinline__ void general_call64(const Args64 &a, long long c)
+{
+    general_node64<KIND, STAGE, ENO3>(a, c);
+}
+
+constexpr int BY64 = 4;  // columns per block (128 threads)
+
+template <int KIND, int STAGE, bool ENO3>
+__global__ void __launch_bounds__(BX *BY64, 4) k_stage64(const __grid_constant__ Args64 a)
+{
+    const Grid &g = a.g;
+    unsigned b = blockIdx.x;
+    if constexpr (band_kind64(KIND)) {
+        // the band blocks come first: their chains are the longest
+        if (b < (unsigned)a.band_blocks) {
+            const unsigned nt = BX * BY64, n = *a.st.flagged.count;
+            for (unsigned t = b * nt + threadIdx.y * BX + threadIdx.x; t < n; t += (unsigned)a.band_blocks * nt)
+                general_node64<KIND, STAGE, ENO3>(a, a.st.flagged.idx[t]);
+            return;
+        }
+        b -= (unsigned)a.band_blocks;
+    }
+    const unsigned nx = (unsigned)(g.rows + BX - 1) / BX, ny = (unsigned)(g.cols + BY64 - 1) / BY64;
+    const unsigned bz = b / (nx * ny), by = (b - bz * nx * ny) / nx, bx = b - (bz * ny + by) * nx;
+    const int i = (int)(bx * BX + threadIdx.x), j = (int)(by * BY64 + threadIdx.y), k = (int)bz;
+    if (i >= g.rows || j >= g.cols) return;
+    const long long c = node_index(g, i, j, k);
+    uint8_t fl = 0;
+    if constexpr (band_kind64(KIND)) {
+        fl = __ldg(a.st.flags + c);
+        if (fl & 0x3F) return;  // a band node
+    }
+    const double ps = __ldg(a.st.phi_s + c);
+    double v[3] = {0.0, 0.0, 0.0};
+    if constexpr (transport_kind64(KIND)) {
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) v[ax] = __ldg(a.st.v.p[ax] + c);
+        if (KIND == K64_ADVECT && a.st.speed) {
+            const double sp = __ldg(a.st.speed + c);
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) v[ax] = sp * v[ax];
+        }
+    }
+    const bool neg = fl & MASK_BIT;
+    // the lines, and whether the short sequences take the node
+    double p[3][7];
+    bool ok = a.ordinary;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        const AxisLine L = axis_line(g, i, j, k, ax);
+#pragma unroll
+        for (int s = 0; s < 7; ++s) {
+            if ((KIND == K64_ENO2 || KIND == K64_ENO2R) && (s == 0 || s == 6)) continue;
+            p[ax][s] = s == 3 ? ps : __ldg(a.st.phi_s + L.base + (long long)clampi(L.c + s - 3, L.n) * L.stride);
+            if (s != 3 || ax == 0) ok = ok && ordinary(p[ax][s]);
+        }
+        // a sign change next to a node without a distance: the general code decides
+        if (KIND == K64_REINIT)
+            ok = ok && ((__double2hiint(p[ax][2]) ^ __double2hiint(ps)) >= 0) &&
+                 ((__double2hiint(p[ax][4]) ^ __double2hiint(ps)) >= 0);
+    }
+    if (!ok) {
+        general_call64<KIND, STAGE, ENO3>(a, c);
+        return;
+    }
+    if constexpr (KIND == K64_VELOCITY) {
+        double n[3];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            const bool fore = fabs(p[ax][4]) < fabs(p[ax][2]);
+            double t[6];
+#pragma unroll
+            for (int m = 0; m < 6; ++m) t[m] = fore ? p[ax][6 - m] : p[ax][m];
+            n[ax] = flip(upwind64(t, a.h[ax], a.rh[ax]), fore);
+        }
+        const double grad = vmax(sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]), a.floor);
+        const double s = ps > 0.0 ? 1.0 : (ps < 0.0 ? -1.0 : 0.0);
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) a.w.p[ax][c] = s * (n[ax] / grad);
+        return;
+    }
+    double step;
+    if constexpr (transport_kind64(KIND)) {
+        // sum_ax min(0, v) D+ + max(0, v) D-: the upwind side alone
+        double tr = 0.0;
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            const bool fore = sign_bit(v[ax]);
+            double D;
+            if constexpr (KIND == K64_ENO2) {
+                const double c2 = __fma_rn(-2.0, ps, p[ax][2]) + p[ax][4];
+                D = eno2_back64(fore ? p[ax][5] : p[ax][1], fore ? p[ax][4] : p[ax][2], ps, c2, a.h[ax], a.rh[ax],
+                                a.h2[ax], a.rh2[ax]);
+            } else {
+                double t[6];
+#pragma unroll
+                for (int m = 0; m < 6; ++m) t[m] = fore ? p[ax][6 - m] : p[ax][m];
+                D = upwind64(t, a.h[ax], a.rh[ax]);
+            }
+            tr = tr + v[ax] * flip(D, fore);
+        }
+        if (KIND == K64_ADVECT)
+            step = __ldg(a.st.dt) * tr;
+        else
+            step = tr * a.dt_uniform;
+    } else {
+        double e[3];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            if constexpr (KIND == K64_ENO2R) {
+                const double c2 = __fma_rn(-2.0, ps, p[ax][2]) + p[ax][4];
+                const double db = eno2_back64(p[ax][1], p[ax][2], ps, c2, a.h[ax], a.rh[ax], a.h2[ax], a.rh2[ax]);
+                const double mf = eno2_back64(p[ax][5], p[ax][4], ps, c2, a.h[ax], a.rh[ax], a.h2[ax], a.rh2[ax]);
+                e[ax] = vmax(0.0, vmax(flip(db, neg), flip(mf, neg)));  // mf = -D+
+            } else {
+                e[ax] = godunov_side64(p[ax], neg, a.h[ax], a.rh[ax]);
+            }
+        }
+        const double gn = norm_root(add_rn(add_rn(sqr(e[0]), sqr(e[1])), sqr(e[2])));
+        step = flip((gn - 1.0) * a.dt_uniform, neg);
+    }
+    if ((KIND == K64_REINIT || KIND == K64_EXTEND) && (fl & FIXED_BIT)) step = 0.0;
+    const double pn = STAGE == 0 ? 0.0 : __ldg(a.st.phi_n + c);
+    if constexpr (KIND == K64_ENO2 || KIND == K64_ENO2R)
+        a.st.out[c] = rk2_combine(STAGE, pn, ps, step);
+    else
+        a.st.out[c] = rk3_combine(STAGE, pn, ps - step);
+}
+
+// ---------------------------------------------------------------------------------------
+// launchers
+// ---------------------------------------------------------------------------------------
+Args64 args64(const Grid &g)
+{
+    Args64 a{};
+    a.g = g;
+    const double h[3] = {g.dx, g.dy, g.dz};
+    a.ordinary = true;
+    for (int q = 0; q < 3; ++q) {
+        a.h[q] = h[q];
+        a.rh[q] = 1.0 / h[q];
+        a.h2[q] = h[q] * h[q];
+        a.rh2[q] = 1.0 / a.h2[q];
+        a.ordinary = a.ordinary && h[q] > std::ldexp(1.0, -60) && h[q] < std::ldexp(1.0, 60);
+    }
+    a.dt_uniform = 0.3 * std::min(std::min(h[0], h[1]), h[2]);
+    return a;
+}
+
+template <int KIND, int STAGE> cudaError_t launch64_as(Args64 &a, bool eno3, cudaStream_t s)
+{
+    const Grid &g = a.g;
+    const long long tiles =
+        (long long)((g.rows + BX - 1) / BX) * ((g.cols + BY64 - 1) / BY64) * g.pges;
+    // band blocks: a node per thread up to four blocks per SM, and no more than the grid has
+    a.band_blocks = band_kind64(KIND) ? (int)std::min<long long>(list_blocks(), tiles) : 0;
+    const unsigned n = (unsigned)(tiles + a.band_blocks);
+    const dim3 bl(BX, BY64);
+    if constexpr (KIND == K64_REINIT || KIND == K64_EXTEND || KIND == K64_VELOCITY) {
+        if (eno3) {
+            k_stage64<KIND, STAGE, true><<<n, bl, 0, s>>>(a);
+            return cudaGetLastError();
+        }
+    }
+    k_stage64<KIND, STAGE, false><<<n, bl, 0, s>>>(a);
+    return cudaGetLastError();
+}
+template <int KIND> cudaError_t launch64(Args64 &a, int stage, bool eno3, cudaStream_t s)
+{
+    if (stage == 0) return launch64_as<KIND, 0>(a, eno3, s);
+    if (stage == 1) return launch64_as<KIND, 1>(a, eno3, s);
+    return launch64_as<KIND, 2>(a, eno3, s);
+}
+
+}  // namespace
+
+cudaError_t launch_stage64(Kind64 kind, bool eno3, const Stage64 &st, int stage, const Grid &g, cudaStream_t s)
+{
+    Args64 a = args64(g);
+    a.st = st;
+    switch (kind) {
+    case K64_REINIT: return launch64<K64_REINIT>(a, stage, eno3, s);
+    case K64_EXTEND: return launch64<K64_EXTEND>(a, stage, eno3, s);
+    case K64_ADVECT: return launch64<K64_ADVECT>(a, stage, eno3, s);
+    case K64_ENO2: return launch64<K64_ENO2>(a, stage, eno3, s);
+    case K64_ENO2R: return launch64<K64_ENO2R>(a, stage, eno3, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template <>
+cudaError_t launch_extension_velocity<double>(const double *phi, const uint8_t *flags, Ptr6<const double> dist,
+                                              Ptr3<double> v, const Grid &g, bool eno3, double floor, NodeList flagged,
+                                              cudaStream_t s)
+{
+    Args64 a = args64(g);
+    a.st.phi_s = phi;
+    a.st.flags = flags;
+    a.st.d = dist;
+    a.st.flagged = flagged;
+    a.w = v;
+    a.floor = floor;
+    return launch64_as<K64_VELOCITY, 0>(a, eno3, s);
+}
+
+}  // namespace vsl

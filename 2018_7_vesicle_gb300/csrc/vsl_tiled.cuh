@@ -1006,6 +1006,20 @@ cudaError_t launch_velocity_tiled(const float *phi, const uint8_t *flags, Ptr3<f
     return cudaGetLastError();
 }
 
+template <>
+cudaError_t launch_extension_velocity<float>(const float *phi, const uint8_t *flags, Ptr6<const float> dist,
+                                             Ptr3<float> v, const Grid &g, bool eno3, double floor, NodeList flagged,
+                                             cudaStream_t s)
+{
+    cudaError_t err = launch_velocity_tiled(phi, flags, v, g, (float)floor, s);
+    if (err != cudaSuccess) return err;
+    if (eno3)
+        k_velocity_list<true><<<list_blocks(), 128, 0, s>>>(phi, flags, dist, v, flagged, g, (float)floor);
+    else
+        k_velocity_list<false><<<list_blocks(), 128, 0, s>>>(phi, flags, dist, v, flagged, g, (float)floor);
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------------------
 // batched stages (k_stage_tiled_batch, k_band_stage_batch)
 // ---------------------------------------------------------------------------------------
