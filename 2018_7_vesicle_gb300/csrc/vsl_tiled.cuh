@@ -32,7 +32,7 @@ namespace {
 
 // Pages per block (a launch parameter: the default below, or the value the tuning table
 // holds for the grid shape and stage kind) and the occupancy target (compile time).
-// Measured on GB300 at 256^3, vesicle step as a graph: 4 blocks per SM (64 registers) beat
+// The default is measured on GB300 at 256^3 (smaller grids: launch_pages), vesicle step as a graph: 4 blocks per SM (64 registers) beat
 // 5 (48 registers with spills) at 16/32/64 pages; with the page loop unrolled by the ring
 // length, 10/15/16/20/25/30/32/40 pages gave 33.6/33.0/33.1/32.7/32.4/32.8/33.0/32.9 ms.
 #ifndef VSL_TILED_KZ
@@ -819,14 +819,57 @@ TileEntry tile_table[TILE_TABLE];
 int tile_count = 0;
 }  // namespace
 
-int tile_pages(const Grid &g, int kind)
+// the table's entry, 0 without one
+static int tile_pages_set(const Grid &g, int kind)
 {
     std::lock_guard<std::mutex> lock(tile_mutex);
     for (int e = 0; e < tile_count; ++e) {
         const TileEntry &t = tile_table[e];
         if (t.rows == g.rows && t.cols == g.cols && t.pges == g.pges && t.kind == kind) return t.pages;
     }
-    return VSL_TILED_KZ;
+    return 0;
+}
+
+int tile_pages(const Grid &g, int kind)
+{
+    const int set = tile_pages_set(g, kind);
+    return set ? set : VSL_TILED_KZ;
+}
+
+
+// Pages per block of a single-grid launch: the tuning table's, else the one of PAGES that the
+// cost below puts lowest.  A block marches its pages at a rate that the blocks resident on its
+// SM share once `share` of them do (fewer leave issue slots idle), and loads planes worth about
+// 1.5 pages before its first one; the busiest SM holds ceil(blocks / SMs) of them.  The page
+// loop is unrolled by five, so counts above five are multiples of it.  The extension keeps the
+// default: on small grids its time is its band blocks' chain, whatever the pages.  Measured on GB300, us per stage, 20 pages / this rule /
+// the best of 1 .. 32: reinitialization 64^3 27.2 / 14.2 / 14.2, 96^3 32.1 / 22.1 / 22.1, 128^3
+// 44.6 / 37.0 / 37.0; ENORK2 extension 64^3 11.0 / 4.7 / 4.7, 96^3 11.5 / 8.8 / 8.1, 128^3 16.8 /
+// 14.4 / 14.2; advection 64^3 11.4 / 5.1 / 5.1, 128^3 21.2 / 21.2 / 20.5.  From about 192^3 on
+// the rule is the default.  (A batch's grids share one launch and keep the default.)
+int launch_pages(const Grid &g, int kind)
+{
+    if (const int set = tile_pages_set(g, kind)) return set;
+    if (kind == SK_EXTEND) return VSL_TILED_KZ;
+    static constexpr int PAGES[] = {1, 2, 3, 4, 5, 10, VSL_TILED_KZ};
+    int share = 4, least = 1;
+    if (kind == SK_ADVECT || kind == SK_VELOCITY) share = 2;
+    if (kind == SK_ENO2) share = 5, least = 4;
+    if (kind == SK_ENO2R) least = 2;
+    const long long sms = list_blocks() / 4;
+    const long long tiles = (long long)((g.rows + TY - 1) / TY) * ((g.cols + TX - 1) / TX);
+    int best = VSL_TILED_KZ;
+    double lowest = 0.0;
+    for (int p : PAGES) {
+        if (p < least) continue;
+        const long long blocks = tiles * ((g.pges + p - 1) / p);
+        const double cost = (p + 1.5) * (double)std::max<long long>(share, (blocks + sms - 1) / sms);
+        if (lowest == 0.0 || cost <= lowest) {
+            lowest = cost;
+            best = p;
+        }
+    }
+    return best;
 }
 
 int set_tile_pages(int rows, int cols, int pges, int kind, int pages)
@@ -961,7 +1004,7 @@ cudaError_t launch_tiled_stage(int kind, bool eno3, const TiledStage &st, const 
         next = st.band.counter + ((st.seq + 1) & 1);
     }
     a.stage = st.stage;
-    a.kz = tile_pages(g, kind);
+    a.kz = launch_pages(g, kind);
     dim3 gr = tiled_grid(g, a.kz), bl(TY, TX);
     if (static_band_kind(kind)) {
         // the static band in the same launch: band blocks after the tile blocks
@@ -1001,7 +1044,7 @@ cudaError_t launch_velocity_tiled(const float *phi, const uint8_t *flags, Ptr3<f
     a.flags = flags;
     a.w = v;
     a.floor = floor;
-    a.kz = tile_pages(g, SK_VELOCITY);
+    a.kz = launch_pages(g, SK_VELOCITY);
     launch_stage_kind<SK_VELOCITY>(0, tiled_grid(g, a.kz), dim3(TY, TX), s, a);
     return cudaGetLastError();
 }
