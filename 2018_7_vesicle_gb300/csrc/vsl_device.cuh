@@ -502,6 +502,57 @@ __device__ __noinline__ void weno_nonuniform_pair(const T xs[7], const T hs[7], 
     d_back = nu_combine(v, c, s);
 }
 
+// One side of weno_nonuniform_pair alone, from the divided differences dd[m] = (hs[m+1] - hs[m]) / (xs[m+1] - xs[m]); the forward one does not
+// read dd[0], the backward one not dd[5].
+template <typename T> __device__ __forceinline__ T weno_nonuniform_fore(const T xs[7], const T dd[6])
+{
+    T e[6], u[5], v[3], c[3], s[3];
+    // forward bias: faces xs[1..6], cells dd[1..5], value at the face xs[3]
+#pragma unroll
+    for (int m = 0; m < 6; ++m) e[m] = xs[m + 1];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) u[m] = dd[m + 1];
+    {
+        const T xm25 = e[0], xm15 = e[1], xm05 = e[2], x05 = e[3], x15 = e[4], x25 = e[5];
+        const T um2 = u[0], um1 = u[1], u0 = u[2], u1 = u[3], u2 = u[4];
+        v[0] = u1 + (u0 - u1) * (T(1.0) + (x05 - xm05) / (x15 - xm05) + (x05 - xm05) / (x25 - xm05)) +
+               (u2 - u1) * ((x05 - xm05) / (x25 - xm05)) * ((x15 - xm05) / (x25 - x05));
+        v[1] = u0 + (um1 - u0) * ((x05 - xm05) / (x15 - xm15)) * ((x15 - xm05) / (x05 - xm15)) -
+               (u1 - u0) * ((x05 - xm05) / (x15 - xm15)) * ((xm05 - xm15) / (x15 - xm05));
+        v[2] = um1 + (u0 - um1) * ((xm05 - xm15) / (x05 - xm25)) * ((xm05 - xm25) / (x05 - xm15)) -
+               (um2 - um1) * ((xm05 - xm15) / (x05 - xm25)) * ((x05 - xm05) / (xm05 - xm25));
+        c[0] = ((xm05 - xm15) / (x25 - xm25)) * ((xm05 - xm25) / (x25 - xm15));
+        c[1] = ((xm05 - xm25) / (x25 - xm25)) * ((x25 - xm05) / (x25 - xm15)) * (T(1.0) + (x25 - xm15) / (x15 - xm25));
+        c[2] = ((x15 - xm05) / (x25 - xm25)) * ((x25 - xm05) / (x15 - xm25));
+    }
+    nu_smoothness(e, u, s);
+    return nu_combine(v, c, s);
+}
+template <typename T> __device__ __forceinline__ T weno_nonuniform_back(const T xs[7], const T dd[6])
+{
+    T e[6], u[5], v[3], c[3], s[3];
+    // backward bias: faces xs[0..5], cells dd[0..4], value at the face xs[3]
+#pragma unroll
+    for (int m = 0; m < 6; ++m) e[m] = xs[m];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) u[m] = dd[m];
+    {
+        const T xm25 = e[0], xm15 = e[1], xm05 = e[2], x05 = e[3], x15 = e[4], x25 = e[5];
+        const T um2 = u[0], um1 = u[1], u0 = u[2], u1 = u[3], u2 = u[4];
+        v[0] = u1 + (u0 - u1) * ((x15 - x05) / (x25 - xm05)) * ((x25 - x05) / (x15 - xm05)) -
+               (u2 - u1) * ((x15 - x05) / (x25 - xm05)) * ((x05 - xm05) / (x25 - x05));
+        v[1] = u0 + (u1 - u0) * ((x05 - xm05) / (x15 - xm15)) * ((x05 - xm15) / (x15 - xm05)) -
+               (um1 - u0) * ((x05 - xm05) / (x15 - xm15)) * ((x15 - x05) / (x05 - xm15));
+        v[2] = um1 + (um2 - um1) * ((x05 - xm05) / (xm05 - xm25)) * ((x05 - xm15) / (x05 - xm25)) +
+               (u0 - um1) * (T(1.0) + (x05 - xm05) / (x05 - xm15) + (x05 - xm05) / (x05 - xm25));
+        c[0] = ((x05 - xm25) / (x25 - xm25)) * ((x05 - xm15) / (x25 - xm15));
+        c[1] = ((x05 - xm25) / (x25 - xm25)) * ((x25 - x05) / (x25 - xm15)) * (T(1.0) + (x25 - xm15) / (x15 - xm25));
+        c[2] = ((x15 - x05) / (x25 - xm25)) * ((x25 - x05) / (x15 - xm25));
+    }
+    nu_smoothness(e, u, s);
+    return nu_combine(v, c, s);
+}
+
 // Nonuniform cubic ENO forward/backward derivatives at xs[3] = 0, the "ENO3" scheme
 // (ENO_cubic_derivative, weno_rk3_reinitialization.cu:189-222).
 template <typename T>
@@ -671,6 +722,43 @@ __device__ __noinline__ void weno_nonuniform_pair_dd(const T G[6], const T dd[6]
         nu_smoothness_gaps(D, u, s);
         d_back = nu_combine(v, c, s);
     }
+}
+
+// one side of weno_nonuniform_pair_dd alone (the forward one does not read dd[0], the backward
+// one not dd[5])
+template <typename T> __device__ __forceinline__ T weno_nonuniform_fore_dd(const T G[6], const T dd[6])
+{
+    T u[5], v[3], c[3], s[3];
+    // forward bias: faces xs[1..6], cells dd[1..5]
+    const FaceSpan<T> D(G + 1);
+#pragma unroll
+    for (int m = 0; m < 5; ++m) u[m] = dd[m + 1];
+    const T um2 = u[0], um1 = u[1], u0 = u[2], u1 = u[3], u2 = u[4];
+    v[0] = u1 + (u0 - u1) * (T(1.0) + D.d23 / D.d24 + D.d23 / D.d25) + (u2 - u1) * (D.d23 / D.d25) * (D.d24 / D.d35);
+    v[1] = u0 + (um1 - u0) * (D.d23 / D.d14) * (D.d24 / D.d13) - (u1 - u0) * (D.d23 / D.d14) * (D.d12 / D.d24);
+    v[2] = um1 + (u0 - um1) * (D.d12 / D.d03) * (D.d02 / D.d13) - (um2 - um1) * (D.d12 / D.d03) * (D.d23 / D.d02);
+    c[0] = (D.d12 / D.d05) * (D.d02 / D.d15);
+    c[1] = (D.d02 / D.d05) * (D.d25 / D.d15) * (T(1.0) + D.d15 / D.d04);
+    c[2] = (D.d24 / D.d05) * (D.d25 / D.d04);
+    nu_smoothness_gaps(D, u, s);
+    return nu_combine(v, c, s);
+}
+template <typename T> __device__ __forceinline__ T weno_nonuniform_back_dd(const T G[6], const T dd[6])
+{
+    T u[5], v[3], c[3], s[3];
+    // backward bias: faces xs[0..5], cells dd[0..4]
+    const FaceSpan<T> D(G);
+#pragma unroll
+    for (int m = 0; m < 5; ++m) u[m] = dd[m];
+    const T um2 = u[0], um1 = u[1], u0 = u[2], u1 = u[3], u2 = u[4];
+    v[0] = u1 + (u0 - u1) * (D.d34 / D.d25) * (D.d35 / D.d24) - (u2 - u1) * (D.d34 / D.d25) * (D.d23 / D.d35);
+    v[1] = u0 + (u1 - u0) * (D.d23 / D.d14) * (D.d13 / D.d24) - (um1 - u0) * (D.d23 / D.d14) * (D.d34 / D.d13);
+    v[2] = um1 + (um2 - um1) * (D.d23 / D.d02) * (D.d13 / D.d03) + (u0 - um1) * (T(1.0) + D.d23 / D.d13 + D.d23 / D.d03);
+    c[0] = (D.d03 / D.d05) * (D.d13 / D.d15);
+    c[1] = (D.d03 / D.d05) * (D.d35 / D.d15) * (T(1.0) + D.d15 / D.d04);
+    c[2] = (D.d34 / D.d05) * (D.d35 / D.d04);
+    nu_smoothness_gaps(D, u, s);
+    return nu_combine(v, c, s);
 }
 
 // eno3_nonuniform_pair on the gaps G[m] = xs[m+1] - xs[m] and the divided differences

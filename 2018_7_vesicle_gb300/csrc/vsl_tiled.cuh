@@ -24,6 +24,7 @@
 #include <cudaTypedefs.h>
 #include <mutex>
 
+#include "vsl_band.cuh"
 #include "vsl_fused.cuh"
 #include "vsl_tma.cuh"
 
@@ -465,6 +466,45 @@ __device__ __forceinline__ double shadow_or(const BandShadow &sh, const uint8_t 
     return (__ldg(flags + n) & 0x3F) ? __ldg(sh.s_in + n) : (double)v;
 }
 
+// The six differences of the line hs[0..6] of an extension band node next to a crossing, in
+// FP64 where an end is an FP64 value: pv, with the node's shadow cs at 3, and on each side with
+// a crossing (right / left) the crossing value (4 / 2) and the shadow of the neighbour beyond it
+// (5 / 1).  The digits cancel in those differences; the quotients are FP32.  A segment between
+// two FP32 values takes the FP32 difference instead: the FP64 difference of two FP32 values is
+// exact unless their exponents lie more than 28 apart, and then it lies far from an FP32
+// rounding boundary, so rounded to FP32 it is the FP32 difference.  Same bits, with 4 of the 6
+// segments in FP64 on a one-sided crossing (FP64 runs at 1/64 of the FP32 rate here).
+__device__ __forceinline__ void extension_differences(const TiledArgs &a, const BandShadow &sh, long long c,
+                                                      const AxisLine &L, int ax, bool right, bool left, double cs,
+                                                      const float p[7], const float pv[7], float dd[6])
+{
+    const bool rs = right, both = rs && left;
+    // the side with the crossing (the right one when both have one): the chain
+    // e0 .. e4 = hs[2..6] (right) or hs[0..4] (left) and its four segments
+    const double cx = __ldg(sh.cp.p[rs ? 2 * ax : 2 * ax + 1] + c);
+    const double sn = shadow_or(sh, a.flags, rs ? c + L.stride : c - L.stride, rs ? p[4] : p[2]);
+    double e0 = (double)(rs ? pv[2] : pv[0]);
+    float x0 = 0.f, x1 = 0.f;  // both sides: segments 0 and 1 in FP64 as well
+    if (both) {
+        const double cl = __ldg(sh.cp.p[2 * ax + 1] + c);
+        const double sl = shadow_or(sh, a.flags, c - L.stride, p[2]);
+        x0 = (float)(sl - (double)pv[0]);
+        x1 = (float)(cl - sl);
+        e0 = cl;
+    }
+    const double e1 = rs ? cs : sn, e3 = rs ? sn : cs, e4 = (double)(rs ? pv[6] : pv[4]);
+    const float f0 = (float)(e1 - e0), f1 = (float)(cx - e1), f2 = (float)(e3 - cx), f3 = (float)(e4 - e3);
+    // the other side's two segments, between FP32 values
+    const float u0 = rs ? pv[0] : pv[4], u1 = rs ? pv[1] : pv[5], u2 = rs ? pv[2] : pv[6];
+    const float g0 = __fsub_rn(u1, u0), g1 = __fsub_rn(u2, u1);
+    dd[0] = rs ? (both ? x0 : g0) : f0;
+    dd[1] = rs ? (both ? x1 : g1) : f1;
+    dd[2] = rs ? f0 : f2;
+    dd[3] = rs ? f1 : f3;
+    dd[4] = rs ? f2 : g0;
+    dd[5] = rs ? f3 : g1;
+}
+
 // one band node of a WENO5 / WENORK3 extension stage (extend_node with the FP64 interface data)
 template <bool ENO3>
 __device__ __forceinline__ void extend_node_mixed(const TiledArgs &a, const BandShadow &sh, int i, int j, int k)
@@ -489,37 +529,8 @@ __device__ __forceinline__ void extend_node_mixed(const TiledArgs &a, const Band
                 crossing_gaps(L, ax, a.d, c, r1, l1, h, rc, lc);
                 float G[6], pv[7];
                 insert_interface_gaps(p, r1, rc, l1, lc, h, 0.f, 0.f, G, pv);
-                // The line hs[0..6] in FP64: pv, with the node's shadow cs at 3, and on each
-                // side with a crossing the crossing value (2 / 4) and the shadow of the
-                // neighbour beyond it (1 / 5).  The differences are taken in FP64 where an
-                // end is such a value (the digits cancel there), the quotients in FP32.  A
-                // segment between two FP32 values takes the FP32 difference instead: the FP64
-                // difference of two FP32 values is exact unless their exponents lie more than
-                // 28 apart, and then it lies far from an FP32 rounding boundary, so rounded to
-                // FP32 it is the FP32 difference.  Same bits, with 4 of the 6 segments in FP64
-                // on a one-sided crossing (FP64 runs at 1/64 of the FP32 rate here).
-                const bool rs = r1 < h, both = rs && l1 < h;
-                // the side with the crossing (the right one when both have one): the chain
-                // e0 .. e4 = hs[2..6] (right) or hs[0..4] (left) and its four segments
-                const double cx = __ldg(sh.cp.p[rs ? 2 * ax : 2 * ax + 1] + c);
-                const double sn = shadow_or(sh, a.flags, rs ? c + L.stride : c - L.stride, rs ? p[4] : p[2]);
-                double e0 = (double)(rs ? pv[2] : pv[0]);
-                float x0 = 0.f, x1 = 0.f;  // both sides: segments 0 and 1 in FP64 as well
-                if (both) {
-                    const double cl = __ldg(sh.cp.p[2 * ax + 1] + c);
-                    const double sl = shadow_or(sh, a.flags, c - L.stride, p[2]);
-                    x0 = (float)(sl - (double)pv[0]);
-                    x1 = (float)(cl - sl);
-                    e0 = cl;
-                }
-                const double e1 = rs ? cs : sn, e3 = rs ? sn : cs, e4 = (double)(rs ? pv[6] : pv[4]);
-                const float f0 = (float)(e1 - e0), f1 = (float)(cx - e1), f2 = (float)(e3 - cx),
-                            f3 = (float)(e4 - e3);
-                // the other side's two segments, between FP32 values
-                const float u0 = rs ? pv[0] : pv[4], u1 = rs ? pv[1] : pv[5], u2 = rs ? pv[2] : pv[6];
-                const float g0 = __fsub_rn(u1, u0), g1 = __fsub_rn(u2, u1);
-                float dd[6] = {rs ? (both ? x0 : g0) : f0, rs ? (both ? x1 : g1) : f1, rs ? f0 : f2,
-                               rs ? f1 : f3, rs ? f2 : g0, rs ? f3 : g1};
+                float dd[6];
+                extension_differences(a, sh, c, L, ax, r1 < h, l1 < h, cs, p, pv, dd);
 #pragma unroll
                 for (int m = 0; m < 6; ++m) dd[m] = dd[m] / G[m];
                 if (ENO3)
@@ -539,6 +550,131 @@ __device__ __forceinline__ void extend_node_mixed(const TiledArgs &a, const Band
     a.out[c] = (float)val;
     sh.s_out[c] = val;
 }
+
+// The band of a WENO5 / WENORK3 extension stage (extend_node with the FP64 interface data) as
+// sorted tasks: per axis the upwind side alone.
+constexpr int EXTEND_CHUNK = 64;  // 192 axes, two thirds of them a half task: one pass of 256 threads
+struct ExtendBand {
+    using Chunk = BandChunk<float, EXTEND_CHUNK>;
+    const TiledArgs &a;
+    __device__ __forceinline__ unsigned node(unsigned t) const { return a.queue[t]; }
+    __device__ __forceinline__ const Grid &grid() const { return a.g; }
+    __device__ __forceinline__ uint8_t flags(unsigned c) const { return __ldg(a.flags + c); }
+    __device__ __forceinline__ unsigned kinds(const Chunk &ch, int node, int ax) const
+    {
+        const float h = a.h[ax];
+        const unsigned c = ch.c[node];
+        const uint8_t fl = ch.fl[node];
+        if (!(flagged_distance(fl, 2 * ax, a.d, c, h) < h || flagged_distance(fl, 2 * ax + 1, a.d, c, h) < h))
+            return 1u << BT_UNIFORM;
+        return __ldg(a.v.p[ax] + c) < 0.f ? 1u << BT_FORE : 1u << BT_BACK;
+    }
+    __device__ __forceinline__ void eval(Chunk &ch, int kind, int node, int ax) const
+    {
+        const unsigned c = ch.c[node];
+        const uint8_t fl = ch.fl[node];
+        const AxisLine L = band_line(ch, a.g, node, ax);
+        const BandShadow &sh = a.sh;
+        float p[7];
+        load_line7(a.phi_s, L, p);
+        const float h = a.h[ax];
+        if (kind == BT_UNIFORM) {
+            float df, db;
+            weno5_pair_fast(p, a.inv_h[ax], a.eps2[ax], df, db);
+            ch.df[ax][node] = df;
+            ch.db[ax][node] = db;
+            return;
+        }
+        const double cs = __ldg(sh.s_in + c);
+        const float r1 = flagged_distance(fl, 2 * ax, a.d, c, h);
+        const float l1 = flagged_distance(fl, 2 * ax + 1, a.d, c, h);
+        float rc, lc;
+        crossing_gaps(L, ax, a.d, c, r1, l1, h, rc, lc);
+        float G[6], pv[7];
+        insert_interface_gaps(p, r1, rc, l1, lc, h, 0.f, 0.f, G, pv);
+        float dd[6];
+        extension_differences(a, sh, c, L, ax, r1 < h, l1 < h, cs, p, pv, dd);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) dd[m] = dd[m] / G[m];
+        const bool back = kind == BT_BACK;
+        const float D = a.eno3 ? nonuniform_side_dd<float, true>(G, dd, back)
+                               : nonuniform_side_dd<float, false>(G, dd, back);
+        (back ? ch.db : ch.df)[ax][node] = D;
+    }
+    __device__ __forceinline__ void finish(const Chunk &ch, int node) const
+    {
+        const unsigned c = ch.c[node];
+        const uint8_t fl = ch.fl[node];
+        const double cs = __ldg(a.sh.s_in + c);
+        float step = 0.f;
+        if (!(fl & FIXED_BIT))
+            step = upwind_dot(__ldg(a.v.p[0] + c), __ldg(a.v.p[1] + c), __ldg(a.v.p[2] + c), ch.df[0][node],
+                              ch.db[0][node], ch.df[1][node], ch.db[1][node], ch.df[2][node], ch.db[2][node]) *
+                   pseudo_dt(fl, a.d, c, a.h[0], a.h[1], a.h[2]);
+        const double pn = a.stage == 0 ? 0.0 : __ldg(a.sh.s_n + c);
+        const double val = rk3_combine(a.stage, pn, cs - (double)step);
+        a.out[c] = (float)val;
+        a.sh.s_out[c] = val;
+    }
+};
+
+// The band of a reinitialization stage (reinit_node) as sorted tasks.
+constexpr int REINIT_CHUNK = 32;  // 96 axes, about 150 tasks: one pass of 128 threads
+template <bool ENO3> struct ReinitBand {
+    using Chunk = BandChunk<float, REINIT_CHUNK>;
+    const TiledArgs &a;
+    __device__ __forceinline__ unsigned node(unsigned t) const { return a.queue[t]; }
+    __device__ __forceinline__ const Grid &grid() const { return a.g; }
+    __device__ __forceinline__ uint8_t flags(unsigned c) const { return __ldg(a.flags + c); }
+    __device__ __forceinline__ unsigned kinds(const Chunk &ch, int node, int ax) const
+    {
+        if (!sign_change(a.phi_s, band_line(ch, a.g, node, ax))) return 1u << BT_UNIFORM;
+        return ENO3 ? 1u << BT_FORE : (1u << BT_FORE) | (1u << BT_BACK);  // the ENO3 pair is one task
+    }
+    __device__ __forceinline__ void eval(Chunk &ch, int kind, int node, int ax) const
+    {
+        const AxisLine L = band_line(ch, a.g, node, ax);
+        float p[7];
+        load_line7(a.phi_s, L, p);
+        const float h = (float)axis_h(a.g, ax);
+        if (kind == BT_UNIFORM) {
+            uniform_pair<float, true>(p, h, ch.df[ax][node], ch.db[ax][node]);
+            return;
+        }
+        const unsigned c = ch.c[node];
+        const uint8_t fl = ch.fl[node];
+        const float r1 = flagged_distance(fl, 2 * ax, a.d, c, h);
+        const float l1 = flagged_distance(fl, 2 * ax + 1, a.d, c, h);
+        float rc, lc;
+        crossing_gaps(L, ax, a.d, c, r1, l1, h, rc, lc);
+        float G[6], hs[7], dd[6];
+        insert_interface_gaps(p, r1, rc, l1, lc, h, 0.f, 0.f, G, hs);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) dd[m] = (hs[m + 1] - hs[m]) / G[m];
+        if constexpr (ENO3) {
+            eno3_nonuniform_pair_dd(G, dd, ch.df[ax][node], ch.db[ax][node]);
+        } else {
+            const bool back = kind == BT_BACK;
+            (back ? ch.db : ch.df)[ax][node] = nonuniform_side_dd<float, false>(G, dd, back);
+        }
+    }
+    __device__ __forceinline__ void finish(const Chunk &ch, int node) const
+    {
+        const unsigned c = ch.c[node];
+        const uint8_t fl = ch.fl[node];
+        const float ps = __ldg(a.phi_s + c);
+        const float hx = (float)a.g.dx, hy = (float)a.g.dy, hz = (float)a.g.dz;
+        float step = 0.f;
+        if (!(fl & FIXED_BIT)) {
+            const bool neg = fl & MASK_BIT;
+            const float gn = godunov_norm(neg, ch.df[0][node], ch.db[0][node], ch.df[1][node], ch.db[1][node],
+                                          ch.df[2][node], ch.db[2][node]);
+            step = (gn - 1.f) * pseudo_dt(fl, a.d, c, hx, hy, hz) * (neg ? -1.f : 1.f);
+        }
+        const float pn = a.stage == 0 ? 0.f : __ldg(a.phi_n + c);
+        a.out[c] = rk3_combine(a.stage, pn, ps - step);
+    }
+};
 
 // one band node of an ENORK2 extension stage (enork2_extend_node with the FP64 interface data)
 __device__ __forceinline__ void enork2_extend_node_mixed(const TiledArgs &a, const BandShadow &sh, int i, int j, int k)
@@ -594,6 +730,15 @@ __device__ __forceinline__ void static_band_node(const TiledArgs &a, long long c
         extend_node_mixed<false>(a, a.sh, i, j, k);
 }
 
+// the static band of a stage, one node per thread, over `nb` blocks of the tiled kernel's shape
+// (this one is block b)
+template <int KIND> __device__ __forceinline__ void static_band(const TiledArgs &a, unsigned b, unsigned nb)
+{
+    const unsigned n = *a.counter;
+    const unsigned t0 = b * (TY * TX) + threadIdx.y * TY + threadIdx.x;
+    for (unsigned t = t0; t < n; t += nb * (TY * TX)) static_band_node<KIND>(a, a.queue[t]);
+}
+
 // The ENORK2 extension kind, whose uniform path is light, is latency-bound at 4 blocks per SM
 // (long-scoreboard stalls, DRAM 35% of peak): 5 blocks (47 registers, no spills) took 100
 // pseudo-steps at 256^3 from 26.7 to 23.6 ms.  The ENORK2 reinitialization was slower at 5
@@ -605,7 +750,9 @@ __device__ __forceinline__ void static_band_node(const TiledArgs &a, long long c
 // update the nodes of the classification's flagged list (grid-stride over the list) instead
 // of a tile.  They are dispatched after the tile blocks and fill the SMs as tile blocks
 // retire, in the same launch; every node still has exactly one writer.
-template <int KIND, int STAGE, bool TMA>
+// TASKS (the extension on grids of up to EXTEND_TASKS_GRID nodes): the band blocks run the list
+// as sorted tasks (vsl_band.cuh) up to EXTEND_TASKS_MOST nodes.
+template <int KIND, int STAGE, bool TMA, bool TASKS = false>
 __global__ void __launch_bounds__(TY *TX, (KIND == SK_ENO2 ? 5 : VSL_TILED_MIN_BLOCKS))
     k_stage_tiled(const __grid_constant__ TiledArgs a, const __grid_constant__ CUtensorMap tm)
 {
@@ -613,12 +760,16 @@ __global__ void __launch_bounds__(TY *TX, (KIND == SK_ENO2 ? 5 : VSL_TILED_MIN_B
     if constexpr (static_band_kind(KIND)) {
         const int bz0 = (int)gridDim.z - a.band_z;
         if ((int)blockIdx.z >= bz0) {
-            const unsigned nt = TY * TX;
             const unsigned nb = gridDim.x * gridDim.y * (unsigned)a.band_z;
             const unsigned b = ((blockIdx.z - (unsigned)bz0) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-            const unsigned n = *a.counter;
-            for (unsigned t = b * nt + threadIdx.y * TY + threadIdx.x; t < n; t += nb * nt)
-                static_band_node<KIND>(a, a.queue[t]);
+            if constexpr (TASKS) {
+                if (*a.counter <= EXTEND_TASKS_MOST) {
+                    __shared__ ExtendBand::Chunk ch;
+                    run_band<TY * TX>(ExtendBand{a}, ch, *a.counter, b, nb, threadIdx.y * TY + threadIdx.x);
+                    return;
+                }
+            }
+            static_band<KIND>(a, b, nb);
             return;
         }
     }
@@ -657,6 +808,14 @@ __global__ void __launch_bounds__(128) k_band_stage(TiledArgs a, unsigned *next_
         const int i = (int)(r - (long long)j * g.rows);
         reinit_node<float, ENO3, true>(a.phi_s, a.phi_n, a.out, a.flags, a.d, g, a.stage, i, j, k);
     }
+}
+// the same band as sorted tasks (vsl_band.cuh), on grids of up to REINIT_TASKS_GRID nodes
+template <bool ENO3>
+__global__ void __launch_bounds__(128) k_band_tasks(const __grid_constant__ TiledArgs a, unsigned *next_counter)
+{
+    if (next_counter && blockIdx.x == 0 && threadIdx.x == 0) *next_counter = 0u;
+    __shared__ typename ReinitBand<ENO3>::Chunk ch;
+    run_band<128>(ReinitBand<ENO3>{a}, ch, *a.counter, blockIdx.x, gridDim.x, threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -712,11 +871,7 @@ __global__ void __launch_bounds__(TY *TX, (KIND == SK_ENO2 ? 5 : VSL_TILED_MIN_B
         if constexpr (static_band_kind(KIND)) {
             // band block of grid v: its static band grid-stride, right after its tiles (its
             // planes still in L2)
-            const TiledArgs &a = B.v[v];
-            const unsigned nt = TY * TX, nb = (unsigned)B.nb[v];
-            const unsigned n = *a.counter;
-            for (unsigned t = (unsigned)(local - B.tiles[v]) * nt + threadIdx.y * TY + threadIdx.x; t < n; t += nb * nt)
-                static_band_node<KIND>(a, a.queue[t]);
+            static_band<KIND>(B.v[v], (unsigned)(local - B.tiles[v]), (unsigned)B.nb[v]);
         }
     }
 }
@@ -842,17 +997,20 @@ int tile_pages(const Grid &g, int kind)
 // SM share once `share` of them do (fewer leave issue slots idle), and loads planes worth about
 // 1.5 pages before its first one; the busiest SM holds ceil(blocks / SMs) of them.  The page
 // loop is unrolled by five, so counts above five are multiples of it.  The extension keeps the
-// default: on small grids its time is its band blocks' chain, whatever the pages.  Measured on GB300, us per stage, 20 pages / this rule /
+// default where its band is not run as tasks: its time is then its band blocks' chain, whatever
+// the pages.  Measured on GB300, us per stage, 20 pages / this rule /
 // the best of 1 .. 32: reinitialization 64^3 27.2 / 14.2 / 14.2, 96^3 32.1 / 22.1 / 22.1, 128^3
 // 44.6 / 37.0 / 37.0; ENORK2 extension 64^3 11.0 / 4.7 / 4.7, 96^3 11.5 / 8.8 / 8.1, 128^3 16.8 /
-// 14.4 / 14.2; advection 64^3 11.4 / 5.1 / 5.1, 128^3 21.2 / 21.2 / 20.5.  From about 192^3 on
+// 14.4 / 14.2; advection 64^3 11.4 / 5.1 / 5.1, 128^3 21.2 / 21.2 / 20.5; WENO5
+// extension (tasks) 64^3 11.5 / 7.7 / 7.5, 96^3 15.9 / 14.4 / 13.5.  From about 192^3 on
 // the rule is the default.  (A batch's grids share one launch and keep the default.)
 int launch_pages(const Grid &g, int kind)
 {
     if (const int set = tile_pages_set(g, kind)) return set;
-    if (kind == SK_EXTEND) return VSL_TILED_KZ;
+    if (kind == SK_EXTEND && g.num > EXTEND_TASKS_GRID) return VSL_TILED_KZ;
     static constexpr int PAGES[] = {1, 2, 3, 4, 5, 10, VSL_TILED_KZ};
     int share = 4, least = 1;
+    if (kind == SK_EXTEND) share = 3, least = 5;
     if (kind == SK_ADVECT || kind == SK_VELOCITY) share = 2;
     if (kind == SK_ENO2) share = 5, least = 4;
     if (kind == SK_ENO2R) least = 2;
@@ -960,6 +1118,17 @@ bool encode_plane_map(CUtensorMap &tm, const float *f, const Grid &g)
 template <int KIND, bool TMA>
 void launch_stage_kind_as(int stage, dim3 gr, dim3 bl, cudaStream_t s, const TiledArgs &a, const CUtensorMap &tm)
 {
+    if constexpr (KIND == SK_EXTEND && !TMA) {
+        if (a.g.num <= EXTEND_TASKS_GRID) {
+            if (stage == 0)
+                k_stage_tiled<KIND, 0, TMA, true><<<gr, bl, 0, s>>>(a, tm);
+            else if (stage == 1)
+                k_stage_tiled<KIND, 1, TMA, true><<<gr, bl, 0, s>>>(a, tm);
+            else
+                k_stage_tiled<KIND, 2, TMA, true><<<gr, bl, 0, s>>>(a, tm);
+            return;
+        }
+    }
     if constexpr (KIND == SK_VELOCITY) {
         k_stage_tiled<KIND, 0, TMA><<<gr, bl, 0, s>>>(a, tm);  // a single pass, not an RK stage
     } else if (stage == 0) {
@@ -1027,6 +1196,13 @@ cudaError_t launch_tiled_stage(int kind, bool eno3, const TiledStage &st, const 
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || kind == SK_ADVECT) return e;
     // the reinitialization's band is queued by the tiled kernel, so its kernel follows it
+    if (g.num <= REINIT_TASKS_GRID) {
+        if (eno3)
+            k_band_tasks<true><<<band_blocks(), 128, 0, s>>>(a, next);
+        else
+            k_band_tasks<false><<<band_blocks(), 128, 0, s>>>(a, next);
+        return cudaGetLastError();
+    }
     if (eno3)
         k_band_stage<true><<<band_blocks(), 128, 0, s>>>(a, next);
     else
