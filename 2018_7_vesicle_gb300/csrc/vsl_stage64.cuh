@@ -17,9 +17,10 @@
 //     sign that the maximum with zero discards (the weights are positive, so the
 //     reconstruction lies between the candidates);
 //   * nodes with an interface distance ("flagged", the classification's list) are updated by
-//     band blocks at the front of the same launch with the general per-node code, so that no
-//     warp of the others runs the nonuniform stencils for a few of its lanes.
-// About 310 / 350 FP64 instructions per node and stage (transport / norm).
+//     band blocks at the front of the same launch, so that no warp of the others runs the
+//     nonuniform stencils for a few of its lanes; the WENO kinds run them as tasks sorted by
+//     stencil kind (vsl_band.cuh), on the same short quotients.
+// About 310 / 350 FP64 instructions per node and stage (transport / norm), the pipe 85% busy.
 //
 // The sequences above need operands away from overflow and underflow.  A node whose stencil
 // holds a value that is neither zero nor of magnitude 2^-400 .. 2^100 (infinities and NaN
@@ -30,6 +31,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "vsl_band.cuh"
 #include "vsl_fused.cuh"
 
 namespace vsl {
@@ -178,6 +180,7 @@ struct Args64 {
     double h[3], rh[3], h2[3], rh2[3];
     double dt_uniform;  // 0.3 * min spacing: the pseudo time step of a node without a flag
     double floor;       // VELOCITY: the floor of |grad phi|
+    double tiny[3];     // 2^-80 h: the least gap of a stencil on short quotients
     bool ordinary;      // the spacings are within the range of the short sequences
 };
 
@@ -208,7 +211,143 @@ template <int KIND, int STAGE, bool ENO3> __device__ __noinline__ void general_c
     general_node64<KIND, STAGE, ENO3>(a, c);
 }
 
-constexpr int BY64 = 4;  // columns per block (128 threads)
+// ---------------------------------------------------------------------------------------
+// the band of the WENO kinds as sorted tasks
+// ---------------------------------------------------------------------------------------
+
+// a double whose quotients are the short ones (operands in their range: see band_line64); the
+// compiler shares the reciprocals of equal divisors
+struct Short64 {
+    double v;
+    __device__ __forceinline__ Short64() {}
+    __device__ __forceinline__ Short64(double x) : v(x) {}
+    friend __device__ __forceinline__ Short64 operator+(Short64 a, Short64 b) { return __dadd_rn(a.v, b.v); }
+    friend __device__ __forceinline__ Short64 operator-(Short64 a, Short64 b) { return __dadd_rn(a.v, -b.v); }
+    friend __device__ __forceinline__ Short64 operator*(Short64 a, Short64 b) { return __dmul_rn(a.v, b.v); }
+    friend __device__ __forceinline__ Short64 operator/(Short64 a, Short64 b) { return quotient(a.v, b.v, reciprocal(b.v)); }
+};
+
+// One side of weno_nonuniform_pair at xs[3].  R: double, or Short64 where every value is ordinary.
+template <typename R> __device__ __forceinline__ double nonuniform_side64(const double xs[7], const double hs[7], bool back)
+{
+    R x[7], dd[6];
+#pragma unroll
+    for (int m = 0; m < 7; ++m) x[m] = R(xs[m]);
+#pragma unroll
+    for (int m = 0; m < 6; ++m) dd[m] = (R(hs[m + 1]) - R(hs[m])) / (x[m + 1] - x[m]);
+    if constexpr (std::is_same<R, double>::value)
+        return back ? weno_nonuniform_back(x, dd) : weno_nonuniform_fore(x, dd);
+    else
+        return back ? weno_nonuniform_back(x, dd).v : weno_nonuniform_fore(x, dd).v;
+}
+__device__ __noinline__ void nonuniform_general64(const double xs[7], const double hs[7], double &df, double &db)
+{
+    weno_nonuniform_pair(xs, hs, df, db);
+}
+
+constexpr int CHUNK64 = 64;  // nodes per chunk: 192 axes over 128 threads
+constexpr int BY64 = 4;      // columns per block (128 threads)
+
+// Ops of run_band for the reinitialization (NORM) and the extension.  The derivatives of both
+// sides are stored where both were evaluated; the Godunov term of a uniform axis
+// (godunov_side64) is stored as the side that the norm takes it from.
+template <int STAGE, bool ENO3, bool NORM> struct Band64 {
+    using Chunk = BandChunk<double, CHUNK64>;
+    const Args64 &a;
+    __device__ __forceinline__ unsigned node(unsigned t) const { return a.st.flagged.idx[t]; }
+    __device__ __forceinline__ const Grid &grid() const { return a.g; }
+    __device__ __forceinline__ uint8_t flags(unsigned c) const { return __ldg(a.st.flags + c); }
+    __device__ __forceinline__ unsigned kinds(const Chunk &ch, int node, int ax) const
+    {
+        const unsigned c = ch.c[node];
+        bool iface;
+        if constexpr (NORM) {
+            iface = sign_change(a.st.phi_s, band_line(ch, a.g, node, ax));
+        } else {
+            const uint8_t fl = ch.fl[node];
+            const double h = a.h[ax];
+            iface = flagged_distance(fl, 2 * ax, a.st.d, c, h) < h || flagged_distance(fl, 2 * ax + 1, a.st.d, c, h) < h;
+        }
+        if (!iface) return 1u << BT_UNIFORM;
+        if (ENO3) return 1u << BT_FORE;  // the ENO3 pair is one task
+        if (NORM) return (1u << BT_FORE) | (1u << BT_BACK);
+        return sign_bit(__ldg(a.st.v.p[ax] + c)) ? 1u << BT_FORE : 1u << BT_BACK;
+    }
+    __device__ __forceinline__ void eval(Chunk &ch, int kind, int node, int ax) const
+    {
+        const unsigned c = ch.c[node];
+        const uint8_t fl = ch.fl[node];
+        const AxisLine L = band_line(ch, a.g, node, ax);
+        double p[7];
+        load_line7(a.st.phi_s, L, p);
+        bool ok = a.ordinary;
+#pragma unroll
+        for (int m = 0; m < 7; ++m) ok = ok && ordinary(p[m]);
+        const double h = a.h[ax];
+        double &df = ch.df[ax][node], &db = ch.db[ax][node];
+        if (kind == BT_UNIFORM) {
+            if (!ok) {
+                weno5_pair_plain(p, h, df, db);
+            } else if constexpr (NORM) {
+                const bool neg = fl & MASK_BIT;
+                (neg ? df : db) = godunov_side64(p, neg, h, a.rh[ax]);
+            } else {
+                const bool fore = sign_bit(__ldg(a.st.v.p[ax] + c));
+                double t[6];
+#pragma unroll
+                for (int m = 0; m < 6; ++m) t[m] = fore ? p[6 - m] : p[m];
+                (fore ? df : db) = flip(upwind64(t, h, a.rh[ax]), fore);
+            }
+            return;
+        }
+        const double r1 = flagged_distance(fl, 2 * ax, a.st.d, c, h);
+        const double l1 = flagged_distance(fl, 2 * ax + 1, a.st.d, c, h);
+        double hf = 0.0, hb = 0.0;
+        if constexpr (!NORM) {
+            hf = r1 < h ? __ldg(a.st.cp.p[2 * ax] + c) : 0.0;
+            hb = l1 < h ? __ldg(a.st.cp.p[2 * ax + 1] + c) : 0.0;
+            ok = ok && ordinary(hf) && ordinary(hb);
+        }
+        double xs[7], hs[7];
+        insert_interface(p, r1, l1, h, hf, hb, xs, hs);
+        if constexpr (ENO3) {
+            eno3_nonuniform_pair(xs, hs, df, db);
+        } else {
+            // gaps below 2^-80 h would leave the range of the short quotients
+            const double tiny = a.tiny[ax];
+            ok = ok && xs[4] > tiny && xs[5] - xs[4] > tiny && -xs[2] > tiny && xs[2] - xs[1] > tiny;
+            const bool back = kind == BT_BACK;
+            if (ok)
+                (back ? db : df) = nonuniform_side64<Short64>(xs, hs, back);
+            else if (NORM)
+                (back ? db : df) = nonuniform_side64<double>(xs, hs, back);
+            else
+                nonuniform_general64(xs, hs, df, db);  // both sides, as the sum reads them
+        }
+    }
+    __device__ __forceinline__ void finish(const Chunk &ch, int node) const
+    {
+        const unsigned c = ch.c[node];
+        const uint8_t fl = ch.fl[node];
+        double step = 0.0;
+        if (!(fl & FIXED_BIT)) {
+            const double dt = pseudo_dt(fl, a.st.d, c, a.h[0], a.h[1], a.h[2]);
+            if constexpr (NORM) {
+                const bool neg = fl & MASK_BIT;
+                const double gn = godunov_norm(neg, ch.df[0][node], ch.db[0][node], ch.df[1][node], ch.db[1][node],
+                                               ch.df[2][node], ch.db[2][node]);
+                step = (gn - 1.0) * dt * (neg ? -1.0 : 1.0);
+            } else {
+                step = upwind_dot(__ldg(a.st.v.p[0] + c), __ldg(a.st.v.p[1] + c), __ldg(a.st.v.p[2] + c),
+                                  ch.df[0][node], ch.db[0][node], ch.df[1][node], ch.db[1][node], ch.df[2][node],
+                                  ch.db[2][node]) *
+                       dt;
+            }
+        }
+        const double pn = STAGE == 0 ? 0.0 : __ldg(a.st.phi_n + c);
+        a.st.out[c] = rk3_combine(STAGE, pn, __ldg(a.st.phi_s + c) - step);
+    }
+};
 
 template <int KIND, int STAGE, bool ENO3>
 __global__ void __launch_bounds__(BX *BY64, 4) k_stage64(const __grid_constant__ Args64 a)
@@ -218,6 +357,13 @@ __global__ void __launch_bounds__(BX *BY64, 4) k_stage64(const __grid_constant__
     if constexpr (band_kind64(KIND)) {
         // the band blocks come first: their chains are the longest
         if (b < (unsigned)a.band_blocks) {
+            if constexpr (KIND == K64_REINIT || KIND == K64_EXTEND) {
+                using Ops = Band64<STAGE, ENO3, KIND == K64_REINIT>;
+                __shared__ typename Ops::Chunk ch;
+                run_band<BX * BY64>(Ops{a}, ch, *a.st.flagged.count, b, (unsigned)a.band_blocks,
+                                    (int)(threadIdx.y * BX + threadIdx.x));
+                return;
+            }
             const unsigned nt = BX * BY64, n = *a.st.flagged.count;
             for (unsigned t = b * nt + threadIdx.y * BX + threadIdx.x; t < n; t += (unsigned)a.band_blocks * nt)
                 general_node64<KIND, STAGE, ENO3>(a, a.st.flagged.idx[t]);
@@ -346,6 +492,7 @@ Args64 args64(const Grid &g)
         a.rh[q] = 1.0 / h[q];
         a.h2[q] = h[q] * h[q];
         a.rh2[q] = 1.0 / a.h2[q];
+        a.tiny[q] = std::ldexp(h[q], -80);
         a.ordinary = a.ordinary && h[q] > std::ldexp(1.0, -60) && h[q] < std::ldexp(1.0, 60);
     }
     a.dt_uniform = 0.3 * std::min(std::min(h[0], h[1]), h[2]);
