@@ -20,7 +20,10 @@
 //     band blocks at the front of the same launch, so that no warp of the others runs the
 //     nonuniform stencils for a few of its lanes; the WENO kinds run them as tasks sorted by
 //     stencil kind (vsl_band.cuh), on the same short quotients.
-// About 310 / 350 FP64 instructions per node and stage (transport / norm), the pipe 85% busy.
+//   * scaled differences are formed once per tile and shared through shared memory.
+// About 280 / 320 FP64 instructions per node and stage (transport / norm), the pipe 85% busy.  Per
+// stage at 128^3 on GB300: advection 1.13 ms, extension 1.23 ms, reinitialization 1.43 ms (3.2,
+// 3.7 and 3.7 ms one node per thread with general quotients).
 //
 // The sequences above need operands away from overflow and underflow.  A node whose stencil
 // holds a value that is neither zero nor of magnitude 2^-400 .. 2^100 (infinities and NaN
@@ -98,24 +101,19 @@ __device__ __forceinline__ double weighted64(double v1, double v2, double v3, do
     return quotient(a1, tot, r) * q[0] + quotient(a2, tot, r) * q[1] + quotient(a3, tot, r) * q[2];
 }
 
-// D- at t[3] of the line t (six points, t[3] the node); the line mirrored about the node
-// gives -D+
-__device__ __forceinline__ double upwind64(const double t[6], double h, double rh)
+// D- from the scaled differences v1..v5 of its window; with the mirrored window of the node's six
+// differences u, upwind64(u[5], u[4], u[3], u[2], u[1]), D+
+__device__ __forceinline__ double upwind64(double v1, double v2, double v3, double v4, double v5)
 {
-    double v[5], q[3];
-#pragma unroll
-    for (int m = 0; m < 5; ++m) v[m] = quotient(t[m + 1] - t[m], h, rh);
-    candidates64(v[0], v[1], v[2], v[3], v[4], q);
-    return weighted64(v[0], v[1], v[2], v[3], v[4], q);
+    double q[3];
+    candidates64(v1, v2, v3, v4, v5, q);
+    return weighted64(v1, v2, v3, v4, v5, q);
 }
 
-// max(0, D-, -D+) of the line p, with both derivatives negated where neg (godunov_norm's
-// term before the square)
-__device__ __forceinline__ double godunov_side64(const double p[7], bool neg, double h, double rh)
+// max(0, D-, -D+) of the scaled differences u of a line, with both derivatives negated where neg
+// (godunov_norm's term before the square)
+__device__ __forceinline__ double godunov_side64(const double u[6], bool neg)
 {
-    double u[6];
-#pragma unroll
-    for (int m = 0; m < 6; ++m) u[m] = quotient(p[m + 1] - p[m], h, rh);
     double qb[3], qf[3];
     {
         const double s1 = 1. / 6. * u[1], s4 = 1. / 6. * u[4], h2 = 1. / 3. * u[2], h3 = 1. / 3. * u[3];
@@ -167,10 +165,6 @@ __device__ __forceinline__ double eno2_back64(double t1, double t2, double t3, d
 // the stage kernel
 // ---------------------------------------------------------------------------------------
 __host__ __device__ constexpr bool band_kind64(int kind) { return kind != K64_ADVECT; }
-__host__ __device__ constexpr bool transport_kind64(int kind)
-{
-    return kind == K64_EXTEND || kind == K64_ADVECT || kind == K64_ENO2;
-}
 
 struct Args64 {
     Stage64 st;
@@ -286,17 +280,18 @@ template <int STAGE, bool ENO3, bool NORM> struct Band64 {
         const double h = a.h[ax];
         double &df = ch.df[ax][node], &db = ch.db[ax][node];
         if (kind == BT_UNIFORM) {
+            double u[6];
+#pragma unroll
+            for (int m = 0; m < 6; ++m) u[m] = quotient(p[m + 1] - p[m], h, a.rh[ax]);
             if (!ok) {
                 weno5_pair_plain(p, h, df, db);
             } else if constexpr (NORM) {
                 const bool neg = fl & MASK_BIT;
-                (neg ? df : db) = godunov_side64(p, neg, h, a.rh[ax]);
+                (neg ? df : db) = godunov_side64(u, neg);
             } else {
                 const bool fore = sign_bit(__ldg(a.st.v.p[ax] + c));
-                double t[6];
-#pragma unroll
-                for (int m = 0; m < 6; ++m) t[m] = fore ? p[6 - m] : p[m];
-                (fore ? df : db) = flip(upwind64(t, h, a.rh[ax]), fore);
+                (fore ? df : db) = upwind64(fore ? u[5] : u[0], fore ? u[4] : u[1], fore ? u[3] : u[2],
+                                            fore ? u[2] : u[3], fore ? u[1] : u[4]);
             }
             return;
         }
@@ -349,133 +344,207 @@ template <int STAGE, bool ENO3, bool NORM> struct Band64 {
     }
 };
 
-template <int KIND, int STAGE, bool ENO3>
-__global__ void __launch_bounds__(BX *BY64, 4) k_stage64(const __grid_constant__ Args64 a)
+// The band blocks at the front of a launch (their chains are the longest); false for a tile block,
+// with b then the tile's number.
+template <int KIND, int STAGE, bool ENO3> __device__ __forceinline__ bool band_block64(const Args64 &a, unsigned &b)
+{
+    if constexpr (!band_kind64(KIND)) return false;
+    if (b >= (unsigned)a.band_blocks) {
+        b -= (unsigned)a.band_blocks;
+        return false;
+    }
+    const unsigned nt = BX * BY64, n = *a.st.flagged.count, tid = threadIdx.y * BX + threadIdx.x;
+    if constexpr (KIND == K64_REINIT || KIND == K64_EXTEND) {
+        using Ops = Band64<STAGE, ENO3, KIND == K64_REINIT>;
+        __shared__ typename Ops::Chunk ch;
+        run_band<BX * BY64>(Ops{a}, ch, n, b, (unsigned)a.band_blocks, (int)tid);
+    } else {
+        for (unsigned t = b * nt + tid; t < n; t += (unsigned)a.band_blocks * nt)
+            general_node64<KIND, STAGE, ENO3>(a, a.st.flagged.idx[t]);
+    }
+    return true;
+}
+
+// The WENO kinds: a block of 32 x 4 threads owns a tile of 32 rows x 4 columns x KZ pages.  Each
+// scaled difference of the tile is formed once, in shared memory (a thread per difference), and
+// read by the five or six nodes whose windows hold it: 28 FP64 instructions per node at KZ = 2
+// instead of 60 (transport) or 72 (norm).  If any value of the tile's stencils is not ordinary,
+// its nodes take the general code.
+template <int KIND, int STAGE, bool ENO3, int KZ>
+__global__ void __launch_bounds__(BX *BY64, 4) k_weno64(const __grid_constant__ Args64 a)
 {
     const Grid &g = a.g;
     unsigned b = blockIdx.x;
-    if constexpr (band_kind64(KIND)) {
-        // the band blocks come first: their chains are the longest
-        if (b < (unsigned)a.band_blocks) {
-            if constexpr (KIND == K64_REINIT || KIND == K64_EXTEND) {
-                using Ops = Band64<STAGE, ENO3, KIND == K64_REINIT>;
-                __shared__ typename Ops::Chunk ch;
-                run_band<BX * BY64>(Ops{a}, ch, *a.st.flagged.count, b, (unsigned)a.band_blocks,
-                                    (int)(threadIdx.y * BX + threadIdx.x));
-                return;
-            }
-            const unsigned nt = BX * BY64, n = *a.st.flagged.count;
-            for (unsigned t = b * nt + threadIdx.y * BX + threadIdx.x; t < n; t += (unsigned)a.band_blocks * nt)
-                general_node64<KIND, STAGE, ENO3>(a, a.st.flagged.idx[t]);
-            return;
-        }
-        b -= (unsigned)a.band_blocks;
+    if (band_block64<KIND, STAGE, ENO3>(a, b)) return;
+    const unsigned nx = (unsigned)(g.rows + BX - 1) / BX, ny = (unsigned)(g.cols + BY64 - 1) / BY64;
+    const unsigned bz = b / (nx * ny), by = (b - bz * nx * ny) / nx, bx = b - (bz * ny + by) * nx;
+    const int i0 = (int)bx * BX, j0 = (int)by * BY64, k0 = (int)bz * KZ;
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * BX + tx;
+    // differences along x between columns j0 + q - 3 and j0 + q - 2, along y between rows
+    // i0 + q - 3 and i0 + q - 2, along z between pages k0 + q - 3 and k0 + q - 2 (all clamped)
+    constexpr int NX = BY64 + 5, NY = BX + 5, NZ = KZ + 5;
+    __shared__ double ux[KZ][NX][BX], uy[KZ][BY64][NY], uz[NZ][BY64][BX];
+    const unsigned rows = (unsigned)g.rows, plane = (unsigned)g.plane;
+    auto at = [&](int i, int j, int k) {
+        return __ldg(a.st.phi_s + ((unsigned)clampi(k, g.pges) * plane + (unsigned)clampi(j, g.cols) * rows +
+                                   (unsigned)clampi(i, g.rows)));
+    };
+    bool ok = a.ordinary;
+    auto scaled = [&](double lo, double hi, int ax) {
+        ok = ok && ordinary(lo) && ordinary(hi);
+        return quotient(hi - lo, a.h[ax], a.rh[ax]);
+    };
+#pragma unroll 1
+    for (int r = ty; r < KZ * NX; r += BY64) {
+        const int kk = r / NX, q = r - kk * NX;
+        ux[kk][q][tx] = scaled(at(i0 + tx, j0 + q - 3, k0 + kk), at(i0 + tx, j0 + q - 2, k0 + kk), AX_X);
     }
+#pragma unroll 1
+    for (int e = tid; e < KZ * BY64 * NY; e += BX * BY64) {
+        const int r = e / NY, q = e - r * NY, kk = r / BY64, jj = r - kk * BY64;
+        uy[kk][jj][q] = scaled(at(i0 + q - 3, j0 + jj, k0 + kk), at(i0 + q - 2, j0 + jj, k0 + kk), AX_Y);
+    }
+#pragma unroll 1
+    for (int q = 0; q < NZ; ++q)
+        uz[q][ty][tx] = scaled(at(i0 + tx, j0 + ty, k0 + q - 3), at(i0 + tx, j0 + ty, k0 + q - 2), AX_Z);
+    ok = __syncthreads_and(ok);
+    const int i = i0 + tx, j = j0 + ty;
+    if (i >= g.rows || j >= g.cols) return;
+#pragma unroll 1
+    for (int kk = 0; kk < KZ && k0 + kk < g.pges; ++kk) {
+        const int k = k0 + kk;
+        const long long c = node_index(g, i, j, k);
+        uint8_t fl = 0;
+        if constexpr (band_kind64(KIND)) {
+            fl = __ldg(a.st.flags + c);
+            if (fl & 0x3F) continue;  // a band node
+        }
+        bool general = !ok;
+        const double ps = __ldg(a.st.phi_s + c);
+        if constexpr (KIND == K64_REINIT) {
+            // a sign change next to a node without a distance: the general code decides
+            const int hi = __double2hiint(ps);
+            general = general || (hi ^ __double2hiint(at(i - 1, j, k))) < 0 || (hi ^ __double2hiint(at(i + 1, j, k))) < 0 ||
+                      (hi ^ __double2hiint(at(i, j - 1, k))) < 0 || (hi ^ __double2hiint(at(i, j + 1, k))) < 0 ||
+                      (hi ^ __double2hiint(at(i, j, k - 1))) < 0 || (hi ^ __double2hiint(at(i, j, k + 1))) < 0;
+        }
+        if (general) {
+            general_call64<KIND, STAGE, ENO3>(a, c);
+            continue;
+        }
+        auto diff = [&](int ax, int m) {
+            return ax == AX_X ? ux[kk][ty + m][tx] : (ax == AX_Y ? uy[kk][ty][tx + m] : uz[kk + m][ty][tx]);
+        };
+        const bool neg = fl & MASK_BIT;
+        double step = 0.0;
+        if constexpr (KIND == K64_REINIT) {
+            double e[3];
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                double u[6];
+#pragma unroll
+                for (int m = 0; m < 6; ++m) u[m] = diff(ax, m);
+                e[ax] = godunov_side64(u, neg);
+            }
+            const double gn = norm_root(add_rn(add_rn(sqr(e[0]), sqr(e[1])), sqr(e[2])));
+            step = flip((gn - 1.0) * a.dt_uniform, neg);
+        } else {
+            // one side of each axis: the upwind one of a transport, sum_ax min(0, v) D+ + max(0, v) D-,
+            // or the one toward the smaller neighbour of the extension velocity
+            double tr = 0.0, n[3];
+            const double sp = KIND == K64_ADVECT && a.st.speed ? __ldg(a.st.speed + c) : 1.0;
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                double v = 0.0;
+                bool fore;
+                if constexpr (KIND == K64_VELOCITY) {
+                    const double pm = at(i - (ax == AX_Y), j - (ax == AX_X), k - (ax == AX_Z));
+                    const double pp = at(i + (ax == AX_Y), j + (ax == AX_X), k + (ax == AX_Z));
+                    fore = fabs(pp) < fabs(pm);
+                } else {
+                    v = __ldg(a.st.v.p[ax] + c);
+                    if (KIND == K64_ADVECT && a.st.speed) v = sp * v;
+                    fore = sign_bit(v);
+                }
+                // the window by index arithmetic: u[0..4], or u[5..1]
+                const int o = fore ? 5 : 0, d = fore ? -1 : 1;
+                n[ax] = upwind64(diff(ax, o), diff(ax, o + d), diff(ax, o + 2 * d), diff(ax, o + 3 * d), diff(ax, o + 4 * d));
+                tr = tr + v * n[ax];
+            }
+            if constexpr (KIND == K64_VELOCITY) {
+                const double grad = vmax(sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]), a.floor);
+                const double s = ps > 0.0 ? 1.0 : (ps < 0.0 ? -1.0 : 0.0);
+#pragma unroll
+                for (int ax = 0; ax < 3; ++ax) a.w.p[ax][c] = s * (n[ax] / grad);
+                continue;
+            }
+            step = KIND == K64_ADVECT ? __ldg(a.st.dt) * tr : tr * a.dt_uniform;
+        }
+        if (band_kind64(KIND) && (fl & FIXED_BIT)) step = 0.0;
+        const double pn = STAGE == 0 ? 0.0 : __ldg(a.st.phi_n + c);
+        a.st.out[c] = rk3_combine(STAGE, pn, ps - step);
+    }
+}
+
+// The ENORK2 kinds: one node per thread.
+template <int KIND, int STAGE>
+__global__ void __launch_bounds__(BX *BY64, 4) k_eno64(const __grid_constant__ Args64 a)
+{
+    const Grid &g = a.g;
+    unsigned b = blockIdx.x;
+    if (band_block64<KIND, STAGE, false>(a, b)) return;
     const unsigned nx = (unsigned)(g.rows + BX - 1) / BX, ny = (unsigned)(g.cols + BY64 - 1) / BY64;
     const unsigned bz = b / (nx * ny), by = (b - bz * nx * ny) / nx, bx = b - (bz * ny + by) * nx;
     const int i = (int)(bx * BX + threadIdx.x), j = (int)(by * BY64 + threadIdx.y), k = (int)bz;
     if (i >= g.rows || j >= g.cols) return;
     const long long c = node_index(g, i, j, k);
-    uint8_t fl = 0;
-    if constexpr (band_kind64(KIND)) {
-        fl = __ldg(a.st.flags + c);
-        if (fl & 0x3F) return;  // a band node
-    }
+    const uint8_t fl = __ldg(a.st.flags + c);
+    if (fl & 0x3F) return;  // a band node
     const double ps = __ldg(a.st.phi_s + c);
-    double v[3] = {0.0, 0.0, 0.0};
-    if constexpr (transport_kind64(KIND)) {
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) v[ax] = __ldg(a.st.v.p[ax] + c);
-        if (KIND == K64_ADVECT && a.st.speed) {
-            const double sp = __ldg(a.st.speed + c);
-#pragma unroll
-            for (int ax = 0; ax < 3; ++ax) v[ax] = sp * v[ax];
-        }
-    }
-    const bool neg = fl & MASK_BIT;
-    // the lines, and whether the short sequences take the node
-    double p[3][7];
-    bool ok = a.ordinary;
+    bool ok = a.ordinary && ordinary(ps);
+    double p[3][7];  // of each line the points 1 .. 5
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
         const AxisLine L = axis_line(g, i, j, k, ax);
 #pragma unroll
-        for (int s = 0; s < 7; ++s) {
-            if ((KIND == K64_ENO2 || KIND == K64_ENO2R) && (s == 0 || s == 6)) continue;
+        for (int s = 1; s < 6; ++s) {
             p[ax][s] = s == 3 ? ps : __ldg(a.st.phi_s + L.base + (long long)clampi(L.c + s - 3, L.n) * L.stride);
-            if (s != 3 || ax == 0) ok = ok && ordinary(p[ax][s]);
+            if (s != 3) ok = ok && ordinary(p[ax][s]);
         }
-        // a sign change next to a node without a distance: the general code decides
-        if (KIND == K64_REINIT)
-            ok = ok && ((__double2hiint(p[ax][2]) ^ __double2hiint(ps)) >= 0) &&
-                 ((__double2hiint(p[ax][4]) ^ __double2hiint(ps)) >= 0);
     }
     if (!ok) {
-        general_call64<KIND, STAGE, ENO3>(a, c);
-        return;
-    }
-    if constexpr (KIND == K64_VELOCITY) {
-        double n[3];
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            const bool fore = fabs(p[ax][4]) < fabs(p[ax][2]);
-            double t[6];
-#pragma unroll
-            for (int m = 0; m < 6; ++m) t[m] = fore ? p[ax][6 - m] : p[ax][m];
-            n[ax] = flip(upwind64(t, a.h[ax], a.rh[ax]), fore);
-        }
-        const double grad = vmax(sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]), a.floor);
-        const double s = ps > 0.0 ? 1.0 : (ps < 0.0 ? -1.0 : 0.0);
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) a.w.p[ax][c] = s * (n[ax] / grad);
+        general_call64<KIND, STAGE, false>(a, c);
         return;
     }
     double step;
-    if constexpr (transport_kind64(KIND)) {
-        // sum_ax min(0, v) D+ + max(0, v) D-: the upwind side alone
+    if constexpr (KIND == K64_ENO2) {
+        // the upwind side alone
         double tr = 0.0;
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
-            const bool fore = sign_bit(v[ax]);
-            double D;
-            if constexpr (KIND == K64_ENO2) {
-                const double c2 = __fma_rn(-2.0, ps, p[ax][2]) + p[ax][4];
-                D = eno2_back64(fore ? p[ax][5] : p[ax][1], fore ? p[ax][4] : p[ax][2], ps, c2, a.h[ax], a.rh[ax],
-                                a.h2[ax], a.rh2[ax]);
-            } else {
-                double t[6];
-#pragma unroll
-                for (int m = 0; m < 6; ++m) t[m] = fore ? p[ax][6 - m] : p[ax][m];
-                D = upwind64(t, a.h[ax], a.rh[ax]);
-            }
-            tr = tr + v[ax] * flip(D, fore);
+            const double v = __ldg(a.st.v.p[ax] + c);
+            const bool fore = sign_bit(v);
+            const double c2 = __fma_rn(-2.0, ps, p[ax][2]) + p[ax][4];
+            const double D = eno2_back64(fore ? p[ax][5] : p[ax][1], fore ? p[ax][4] : p[ax][2], ps, c2, a.h[ax],
+                                         a.rh[ax], a.h2[ax], a.rh2[ax]);
+            tr = tr + v * flip(D, fore);
         }
-        if (KIND == K64_ADVECT)
-            step = __ldg(a.st.dt) * tr;
-        else
-            step = tr * a.dt_uniform;
+        step = tr * a.dt_uniform;
     } else {
+        const bool neg = fl & MASK_BIT;
         double e[3];
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
-            if constexpr (KIND == K64_ENO2R) {
-                const double c2 = __fma_rn(-2.0, ps, p[ax][2]) + p[ax][4];
-                const double db = eno2_back64(p[ax][1], p[ax][2], ps, c2, a.h[ax], a.rh[ax], a.h2[ax], a.rh2[ax]);
-                const double mf = eno2_back64(p[ax][5], p[ax][4], ps, c2, a.h[ax], a.rh[ax], a.h2[ax], a.rh2[ax]);
-                e[ax] = vmax(0.0, vmax(flip(db, neg), flip(mf, neg)));  // mf = -D+
-            } else {
-                e[ax] = godunov_side64(p[ax], neg, a.h[ax], a.rh[ax]);
-            }
+            const double c2 = __fma_rn(-2.0, ps, p[ax][2]) + p[ax][4];
+            const double db = eno2_back64(p[ax][1], p[ax][2], ps, c2, a.h[ax], a.rh[ax], a.h2[ax], a.rh2[ax]);
+            const double mf = eno2_back64(p[ax][5], p[ax][4], ps, c2, a.h[ax], a.rh[ax], a.h2[ax], a.rh2[ax]);
+            e[ax] = vmax(0.0, vmax(flip(db, neg), flip(mf, neg)));  // mf = -D+
         }
         const double gn = norm_root(add_rn(add_rn(sqr(e[0]), sqr(e[1])), sqr(e[2])));
         step = flip((gn - 1.0) * a.dt_uniform, neg);
     }
-    if ((KIND == K64_REINIT || KIND == K64_EXTEND) && (fl & FIXED_BIT)) step = 0.0;
     const double pn = STAGE == 0 ? 0.0 : __ldg(a.st.phi_n + c);
-    if constexpr (KIND == K64_ENO2 || KIND == K64_ENO2R)
-        a.st.out[c] = rk2_combine(STAGE, pn, ps, step);
-    else
-        a.st.out[c] = rk3_combine(STAGE, pn, ps - step);
+    a.st.out[c] = rk2_combine(STAGE, pn, ps, step);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -499,23 +568,37 @@ Args64 args64(const Grid &g)
     return a;
 }
 
-template <int KIND, int STAGE> cudaError_t launch64_as(Args64 &a, bool eno3, cudaStream_t s)
+template <int KIND, int STAGE, int KZ> cudaError_t launch64_weno(Args64 &a, bool eno3, unsigned blocks, cudaStream_t s)
 {
-    const Grid &g = a.g;
-    const long long tiles =
-        (long long)((g.rows + BX - 1) / BX) * ((g.cols + BY64 - 1) / BY64) * g.pges;
-    // band blocks: a node per thread up to four blocks per SM, and no more than the grid has
-    a.band_blocks = band_kind64(KIND) ? (int)std::min<long long>(list_blocks(), tiles) : 0;
-    const unsigned n = (unsigned)(tiles + a.band_blocks);
     const dim3 bl(BX, BY64);
-    if constexpr (KIND == K64_REINIT || KIND == K64_EXTEND || KIND == K64_VELOCITY) {
+    if constexpr (KIND != K64_ADVECT) {
         if (eno3) {
-            k_stage64<KIND, STAGE, true><<<n, bl, 0, s>>>(a);
+            k_weno64<KIND, STAGE, true, KZ><<<blocks, bl, 0, s>>>(a);
             return cudaGetLastError();
         }
     }
-    k_stage64<KIND, STAGE, false><<<n, bl, 0, s>>>(a);
+    k_weno64<KIND, STAGE, false, KZ><<<blocks, bl, 0, s>>>(a);
     return cudaGetLastError();
+}
+template <int KIND, int STAGE> cudaError_t launch64_as(Args64 &a, bool eno3, cudaStream_t s)
+{
+    const Grid &g = a.g;
+    const long long columns = (long long)((g.rows + BX - 1) / BX) * ((g.cols + BY64 - 1) / BY64);
+    // band blocks: up to four per SM, and no more than the grid has nodes for
+    a.band_blocks = band_kind64(KIND) ? (int)std::min<long long>(list_blocks(), columns * g.pges) : 0;
+    if constexpr (KIND == K64_ENO2 || KIND == K64_ENO2R) {
+        k_eno64<KIND, STAGE><<<(unsigned)(columns * g.pges + a.band_blocks), dim3(BX, BY64), 0, s>>>(a);
+        return cudaGetLastError();
+    } else {
+        // Two pages per block where that leaves twelve blocks per SM, else one (a whole-SM imbalance
+        // then costs more than the z differences saved).  Measured on GB300, ms, one / two / four
+        // pages: 10 WENO5 reinitialization pseudo-steps 32^3 2.02 / 2.15 / 3.03, 64^3 6.63 / 6.82 /
+        // 7.67, 96^3 19.6 / 19.4 / 19.9, 128^3 43.8 / 42.9 / 43.0; 10 extension pseudo-steps 96^3
+        // 16.5 / 16.2 / 16.0, 128^3 37.8 / 36.8 / 36.3 (each difference formed per node: 47.9, 40.6).
+        const long long tall = columns * ((g.pges + 1) / 2);
+        if (tall >= 3 * list_blocks()) return launch64_weno<KIND, STAGE, 2>(a, eno3, (unsigned)(tall + a.band_blocks), s);
+        return launch64_weno<KIND, STAGE, 1>(a, eno3, (unsigned)(columns * g.pges + a.band_blocks), s);
+    }
 }
 template <int KIND> cudaError_t launch64(Args64 &a, int stage, bool eno3, cudaStream_t s)
 {
