@@ -44,7 +44,7 @@ __device__ __forceinline__ bool a_node(const Grid &g, int &i, int &j, int &k, lo
 }
 
 // F's toolbox values at one node: gradient, |grad F| (floored), Hessian, normal, and the
-// Heaviside function from the primal max(F, 0) -- k_toolbox's expressions in its order
+// Heaviside function from the primal max(F, 0) -- tool64_node's expressions in its order
 template <typename T> struct FPart {
     T fx, fy, fz, gm, nx, ny, nz, fxx, fyy, fzz, fxy, fyz, fzx, heav;
 };

@@ -3,6 +3,7 @@
 // (cited per kernel) with the same arithmetic; the neighbour gathers use 64-bit clamped
 // indices and read-only loads.
 #include "vsl_internal.h"
+#include "vsl_tool64.cuh"
 
 namespace vsl {
 namespace {
@@ -208,57 +209,53 @@ struct Fields18 {
     double *p[18];
 };
 
-__global__ void __launch_bounds__(BX *BY) k_set_calculus_toolbox(Fields18 o, const double *__restrict__ f,
-                                                                   const double *__restrict__ hp, Grid g, double ds)
+template <typename R>
+__device__ __forceinline__ void toolbox_node(const Fields18 &o, const double *__restrict__ f,
+                                             const double *__restrict__ hp, const Grid &g, const Tool64 &t, int i, int j,
+                                             int k, long long c)
+{
+    auto at = [&](const double *q, int a, int b, int e) { return __ldg(q + node_index(g, a, b, e)); };
+    double v[18];
+    tool64_node<R>([&](int a, int b, int e) { return at(f, a, b, e); }, [&](int a, int b, int e) { return at(hp, a, b, e); },
+                   i, j, k, clampi(i - 1, g.rows), clampi(i + 1, g.rows), clampi(j - 1, g.cols), clampi(j + 1, g.cols),
+                   clampi(k - 1, g.pges), clampi(k + 1, g.pges), t, TOOL_ALL, v);
+#pragma unroll
+    for (int q = 0; q < 18; ++q) o.p[q][c] = v[q];
+}
+__device__ __noinline__ void toolbox_general(const Fields18 &o, const double *__restrict__ f,
+                                             const double *__restrict__ hp, const Grid &g, const Tool64 &t, int i, int j,
+                                             int k, long long c)
+{
+    toolbox_node<double>(o, f, hp, g, t, i, j, k, c);
+}
+// Bound by the FP64 pipe (about 310 FP64 instructions per node, 560 with general divisions).
+__global__ void __launch_bounds__(BX *BY) k_set_calculus_toolbox(const __grid_constant__ Fields18 o,
+                                                                 const double *__restrict__ f,
+                                                                 const double *__restrict__ hp,
+                                                                 const __grid_constant__ Grid g,
+                                                                 const __grid_constant__ Tool64 t)
 {
     int i, j, k;
     if (!node_of_thread(g, i, j, k)) return;
     const long long c = node_index(g, i, j, k);
-    const long long xp = clamped_index(g, i, j + 1, k), xm = clamped_index(g, i, j - 1, k);
-    const long long yp = clamped_index(g, i + 1, j, k), ym = clamped_index(g, i - 1, j, k);
-    const long long zp = clamped_index(g, i, j, k + 1), zm = clamped_index(g, i, j, k - 1);
-    const double dx = g.dx, dy = g.dy, dz = g.dz;
-    const double fc = __ldg(f + c);
-    double fx = (__ldg(f + xp) - __ldg(f + xm)) / (2 * dx);
-    double fy = (__ldg(f + yp) - __ldg(f + ym)) / (2 * dy);
-    double fz = (__ldg(f + zp) - __ldg(f + zm)) / (2 * dz);
-    double gm = vmax(sqrt(fx * fx + fy * fy + fz * fz), 1e-14);
-    double fxx = (__ldg(f + xp) - 2 * fc + __ldg(f + xm)) / (dx * dx);
-    double fyy = (__ldg(f + yp) - 2 * fc + __ldg(f + ym)) / (dy * dy);
-    double fzz = (__ldg(f + zp) - 2 * fc + __ldg(f + zm)) / (dz * dz);
-    double fxy = (__ldg(f + clamped_index(g, i + 1, j + 1, k)) + __ldg(f + clamped_index(g, i - 1, j - 1, k)) -
-                  __ldg(f + clamped_index(g, i + 1, j - 1, k)) - __ldg(f + clamped_index(g, i - 1, j + 1, k))) /
-                 (4 * ds * ds);
-    double fyz = (__ldg(f + clamped_index(g, i + 1, j, k + 1)) + __ldg(f + clamped_index(g, i - 1, j, k - 1)) -
-                  __ldg(f + clamped_index(g, i + 1, j, k - 1)) - __ldg(f + clamped_index(g, i - 1, j, k + 1))) /
-                 (4 * ds * ds);
-    double fzx = (__ldg(f + clamped_index(g, i, j + 1, k + 1)) + __ldg(f + clamped_index(g, i, j - 1, k - 1)) -
-                  __ldg(f + clamped_index(g, i, j + 1, k - 1)) - __ldg(f + clamped_index(g, i, j - 1, k + 1))) /
-                 (4 * ds * ds);
-    double lap = fxx + fyy + fzz;
-    double r1 = fxx * fx + fxy * fy + fzx * fz;
-    double r2 = fxy * fx + fyy * fy + fyz * fz;
-    double r3 = fzx * fx + fyz * fy + fzz * fz;
-    double mean = -lap / gm + (fx * r1 + fy * r2 + fz * r3) / pow_cr<3>(gm);
-    r1 = (fyy * fzz - fyz * fyz) * fx + (fzx * fyz - fxy * fzz) * fy + (fxy * fyz - fzx * fyy) * fz;
-    r2 = (fyz * fzx - fxy * fzz) * fx + (fxx * fzz - fzx * fzx) * fy + (fzx * fxy - fxx * fyz) * fz;
-    r3 = (fxy * fyz - fyy * fzx) * fx + (fzx * fxy - fxx * fyz) * fy + (fxx * fyy - fxy * fxy) * fz;
-    double gm2 = gm * gm;
-    const double gm4 = pow_cr<4>(gm);
-    double gauss = (fx * r1 + fy * r2 + fz * r3) / gm4;
-    double px = (__ldg(hp + xp) - __ldg(hp + xm)) / (2 * dx);
-    double py = (__ldg(hp + yp) - __ldg(hp + ym)) / (2 * dy);
-    double pz = (__ldg(hp + zp) - __ldg(hp + zm)) / (2 * dz);
-    double dot = px * fx + py * fy + pz * fz;
-    const double hc = __ldg(hp + c);
-    double pxx = (__ldg(hp + xp) - 2 * hc + __ldg(hp + xm)) / (dx * dx);
-    double pyy = (__ldg(hp + yp) - 2 * hc + __ldg(hp + ym)) / (dy * dy);
-    double pzz = (__ldg(hp + zp) - 2 * hc + __ldg(hp + zm)) / (dz * dz);
-    double plap = pxx + pyy + pzz;
-    const double vals[18] = {fx,  fy,  fz,  gm,  fx / gm, fy / gm, fz / gm, fxx, fyy, fzz, fxy, fyz, fzx, lap, mean,
-                             gauss, dot / gm2, plap / gm2 - dot * lap / gm4};
+    // the short quotients where the node's 19 values and its primal's 7 are ordinary
+    bool ok = t.ordinary;
 #pragma unroll
-    for (int q = 0; q < 18; ++q) o.p[q][c] = vals[q];
+    for (int a = -1; a <= 1; ++a)
+#pragma unroll
+        for (int b = -1; b <= 1; ++b)
+#pragma unroll
+            for (int e = -1; e <= 1; ++e) {
+                const int off = (a != 0) + (b != 0) + (e != 0);
+                if (off > 2) continue;
+                const long long q = clamped_index(g, i + a, j + b, k + e);
+                ok = ok && ordinary_tool(__ldg(f + q));
+                if (off <= 1) ok = ok && ordinary_tool(__ldg(hp + q));
+            }
+    if (ok)
+        toolbox_node<Short64>(o, f, hp, g, t, i, j, k, c);
+    else
+        toolbox_general(o, f, hp, g, t, i, j, k, c);
 }
 
 // ---- ENORK2 (1_0_ENORK2_Reinitialization/boundary_correction.cu,
@@ -636,7 +633,7 @@ int vsl_set_calculus_toolbox(double *Fx, double *Fy, double *Fz, double *FGradMa
     Grid g = make_grid(rows, cols, pges, dx, dy, dz);
     Fields18 o = {{Fx, Fy, Fz, FGradMag, Nx, Ny, Nz, Fxx, Fyy, Fzz, Fxy, Fyz, Fzx, FLaplacian, MeanCurvature,
                    GaussianCurvature, Heaviside, DiracDelta}};
-    k_set_calculus_toolbox<<<node_grid(g), dim3(BX, BY), 0, stream>>>(o, lsf, HPrimal, g, ds);
+    k_set_calculus_toolbox<<<node_grid(g), dim3(BX, BY), 0, stream>>>(o, lsf, HPrimal, g, tool64(g, ds));
     return launch_status(cudaGetLastError());
 }
 

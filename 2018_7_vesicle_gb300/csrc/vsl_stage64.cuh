@@ -6,11 +6,8 @@
 // (loads, integer work, selects) is free beside it.  A node of the per-node form costs about
 // 1100 FP64 instructions per stage: 24 quotients per axis as general divisions, and both
 // one-sided derivatives of every axis.  Here:
-//   * quotients by the grid spacing take its correctly rounded reciprocal (formed on the
-//     host) and the multiply / remainder / correction sequence of Markstein (IBM J. Res.
-//     Dev. 34, 1990): three instructions, the correctly rounded quotient;
-//   * the WENO weights' quotients share one reciprocal per divisor, from the documented PTX
-//     approximation rcp.approx.ftz.f64 and one third-order Newton step (error 1 - b y cubed);
+//   * quotients are the short ones of vsl_short64.cuh: three instructions by the grid spacing,
+//     one shared reciprocal per divisor in the WENO weights;
 //   * multiplications by powers of two ride in an FMA, which rounds the same;
 //   * transport evaluates only the upwind side of an axis (the other is multiplied by zero),
 //     and the Godunov norm only the sides whose three candidate values do not all have the
@@ -36,38 +33,13 @@
 
 #include "vsl_band.cuh"
 #include "vsl_fused.cuh"
+#include "vsl_short64.cuh"
 
 namespace vsl {
 namespace {
 
-// ---------------------------------------------------------------------------------------
-// quotients
-// ---------------------------------------------------------------------------------------
-
-// a / d for the divisor d whose reciprocal r is 1 / d to within an ulp
-__device__ __forceinline__ double quotient(double a, double d, double r)
-{
-    const double q = __dmul_rn(a, r);
-    return __fma_rn(__fma_rn(-d, q, a), r, q);
-}
-
-// 1 / d to within an ulp for a normal d whose reciprocal is normal
-__device__ __forceinline__ double reciprocal(double d)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = __fma_rn(-d, y, 1.0);  // at most about 2^-19
-    return __fma_rn(y, __fma_rn(e, e, e), y);
-}
-
-// magnitude bits of the high word
-__device__ __forceinline__ int mag_hi(double x) { return __double2hiint(x) & 0x7fffffff; }
 // zero, or of magnitude 2^-400 .. 2^100
-__device__ __forceinline__ bool ordinary(double x)
-{
-    const unsigned m = (unsigned)mag_hi(x);
-    return m - (unsigned)((1023 - 400) << 20) < (unsigned)(500 << 20) || (m | (unsigned)__double2loint(x)) == 0u;
-}
+__device__ __forceinline__ bool ordinary(double x) { return within64(x, -400, 100); }
 __device__ __forceinline__ bool sign_bit(double x) { return __double2hiint(x) < 0; }
 __device__ __forceinline__ double flip(double x, bool neg)
 {
@@ -208,18 +180,6 @@ template <int KIND, int STAGE, bool ENO3> __device__ __noinline__ void general_c
 // ---------------------------------------------------------------------------------------
 // the band of the WENO kinds as sorted tasks
 // ---------------------------------------------------------------------------------------
-
-// a double whose quotients are the short ones (operands in their range: see band_line64); the
-// compiler shares the reciprocals of equal divisors
-struct Short64 {
-    double v;
-    __device__ __forceinline__ Short64() {}
-    __device__ __forceinline__ Short64(double x) : v(x) {}
-    friend __device__ __forceinline__ Short64 operator+(Short64 a, Short64 b) { return __dadd_rn(a.v, b.v); }
-    friend __device__ __forceinline__ Short64 operator-(Short64 a, Short64 b) { return __dadd_rn(a.v, -b.v); }
-    friend __device__ __forceinline__ Short64 operator*(Short64 a, Short64 b) { return __dmul_rn(a.v, b.v); }
-    friend __device__ __forceinline__ Short64 operator/(Short64 a, Short64 b) { return quotient(a.v, b.v, reciprocal(b.v)); }
-};
 
 // One side of weno_nonuniform_pair at xs[3].  R: double, or Short64 where every value is ordinary.
 template <typename R> __device__ __forceinline__ double nonuniform_side64(const double xs[7], const double hs[7], bool back)
@@ -562,7 +522,7 @@ Args64 args64(const Grid &g)
         a.h2[q] = h[q] * h[q];
         a.rh2[q] = 1.0 / a.h2[q];
         a.tiny[q] = std::ldexp(h[q], -80);
-        a.ordinary = a.ordinary && h[q] > std::ldexp(1.0, -60) && h[q] < std::ldexp(1.0, 60);
+        a.ordinary = a.ordinary && ordinary_spacing(h[q]);
     }
     a.dt_uniform = 0.3 * std::min(std::min(h[0], h[1]), h[2]);
     return a;

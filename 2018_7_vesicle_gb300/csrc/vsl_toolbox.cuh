@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "vsl_internal.h"
+#include "vsl_tool64.cuh"
 
 namespace vsl {
 namespace {
@@ -39,13 +40,6 @@ __device__ __forceinline__ long long block_linear() { return blockIdx.x + (long 
 // plain form is FP64 throughout; the mixed form computes these stencils in FP32), with
 // HPrimal = max(F, 0) formed on the fly (GPUsetCalculusToolBox.m:4); per block the FP64
 // sums of DiracDelta over |F| < 2Ds and of 1 - Heaviside over F < 2Ds (SDF3.m:73-80).
-template <typename T> __device__ __forceinline__ T cube(T x);
-template <> __device__ __forceinline__ double cube<double>(double x) { return pow_cr<3>(x); }
-template <> __device__ __forceinline__ float cube<float>(float x) { return x * x * x; }
-template <typename T> __device__ __forceinline__ T fourth(T x);
-template <> __device__ __forceinline__ double fourth<double>(double x) { return pow_cr<4>(x); }
-template <> __device__ __forceinline__ float fourth<float>(float x) { return (x * x) * (x * x); }
-
 // reciprocals of the spacings for the mixed form: FP64 for its area and volume terms, FP32
 // for its stencils
 struct Recips {
@@ -86,7 +80,7 @@ __device__ __forceinline__ void band_terms_f64(const float v[8], const Recips &r
     }
 }
 
-// One node of the mixed form's toolbox: the expressions of toolbox_point in FP32 with the
+// One node of the mixed form's toolbox: the expressions of tool64_node in FP32 with the
 // divisions by the spacings as products with their FP32 reciprocals and one reciprocal of
 // |grad F| (the reference's quotients, rounded differently within a few ulp); the fields
 // that only an output needs (Gaussian curvature, Heaviside, Dirac delta) are formed only
@@ -175,130 +169,123 @@ __device__ __forceinline__ bool toolbox_point_f32(Get F, int i, int j, int k, in
     return need;
 }
 
-// One node of the plain FP64 toolbox (set_calculus_toolbox.cu:9-107), the reference's
-// expressions in its order.
+// The plain FP64 toolbox, one node per thread, the reference's expressions (tool64_node).  The
+// area and volume terms need the Heaviside and Dirac functions, which are formed at every node
+// only where an output asks for them; otherwise at the nodes that carry a term (F < 2 Ds with a
+// positive value among the seven; without one the volume term is exactly 1 and the area term 0),
+// listed per block in shared memory and evaluated in full warps: a warp with one such node would
+// otherwise run the FP64 block for all its lanes.  Each term returns to its node's thread, so the
+// sums keep their order: warp shuffle tree, then the block's warps.
+// thr2ds: 2 Ds (the reference's band tests).
 template <class Get>
-__device__ __forceinline__ void toolbox_point_f64(Get F, int i, int j, int k, int im, int ip, int jm, int jp,
-                                                  int km, int kp, long long c, const ToolboxOut<double> &o,
-                                                  const Grid &g, double ds_, double thr2ds, double &area,
-                                                  double &vol, int &units)
+__device__ __noinline__ void tool64_general(Get F, int i, int j, int k, int im, int ip, int jm, int jp, int km, int kp,
+                                            const Tool64 &t, unsigned want, double v[18])
 {
-    using T = double;
-    bool unit = false;
-    auto H = [&](int a, int b, int e) { return vmax(F(a, b, e), T(0)); };
-    const T dx = (T)g.dx, dy = (T)g.dy, dz = (T)g.dz, ds = (T)ds_;
-    const T fc = F(i, j, k);
-    const T fxp = F(i, jp, k), fxm = F(i, jm, k), fyp = F(ip, j, k), fym = F(im, j, k);
-    const T fzp = F(i, j, kp), fzm = F(i, j, km);
-    T fx = (fxp - fxm) / (2 * dx);
-    T fy = (fyp - fym) / (2 * dy);
-    T fz = (fzp - fzm) / (2 * dz);
-    T gm = vmax(sqrt(fx * fx + fy * fy + fz * fz), T(1e-14));
-    T fxx = (fxp - 2 * fc + fxm) / (dx * dx);
-    T fyy = (fyp - 2 * fc + fym) / (dy * dy);
-    T fzz = (fzp - 2 * fc + fzm) / (dz * dz);
-    T fxy = (F(ip, jp, k) + F(im, jm, k) - F(ip, jm, k) - F(im, jp, k)) / (4 * ds * ds);
-    T fyz = (F(ip, j, kp) + F(im, j, km) - F(ip, j, km) - F(im, j, kp)) / (4 * ds * ds);
-    T fzx = (F(i, jp, kp) + F(i, jm, km) - F(i, jp, km) - F(i, jm, kp)) / (4 * ds * ds);
-    T lap = fxx + fyy + fzz;
-    T r1 = fxx * fx + fxy * fy + fzx * fz;
-    T r2 = fxy * fx + fyy * fy + fyz * fz;
-    T r3 = fzx * fx + fyz * fy + fzz * fz;
-    T gm2 = gm * gm;
-    T mean = -lap / gm + (fx * r1 + fy * r2 + fz * r3) / cube(gm);
-    const T gm4 = fourth(gm);
-    T hc = vmax(fc, T(0));
-    T hxp = H(i, jp, k), hxm = H(i, jm, k), hyp = H(ip, j, k), hym = H(im, j, k);
-    T hzp = H(i, j, kp), hzm = H(i, j, km);
-    T px = (hxp - hxm) / (2 * dx), py = (hyp - hym) / (2 * dy), pz = (hzp - hzm) / (2 * dz);
-    T dot = px * fx + py * fy + pz * fz;
-    T pxx = (hxp - 2 * hc + hxm) / (dx * dx);
-    T pyy = (hyp - 2 * hc + hym) / (dy * dy);
-    T pzz = (hzp - 2 * hc + hzm) / (dz * dz);
-    T plap = pxx + pyy + pzz;
-    T heav = dot / gm2;
-    T delta = plap / gm2 - dot * lap / gm4;
-    if (fabs(fc) < thr2ds) area += delta;
-    if (fc < thr2ds) {
-        // heav == 0 (no positive neighbour) gives a volume term of exactly 1
-        if (heav == T(0)) {
-            unit = true;
-        } else {
-            const double v1 = 1 - heav;
+    tool64_node<double>(F, [&](int a, int b, int e) { return vmax(F(a, b, e), 0.0); }, i, j, k, im, ip, jm, jp, km, kp,
+                        t, want, v);
+}
+
+__global__ void __launch_bounds__(NT) k_toolbox64(const double *__restrict__ f, const __grid_constant__ ToolboxOut<double> o,
+                                                  const __grid_constant__ Grid g, double thr2ds,
+                                                  double *__restrict__ partials, const __grid_constant__ Tool64 tc,
+                                                  unsigned want)
+{
+    const int i0 = blockIdx.x * BX, j0 = blockIdx.y * BY, k = blockIdx.z;
+    const int t = threadIdx.y * BX + threadIdx.x;
+    const unsigned rows = (unsigned)g.rows, plane = (unsigned)g.plane;
+    // node offsets in 32 bits (grids hold fewer than 2^31 nodes)
+    auto F = [&](int a, int b, int e) { return __ldg(f + ((unsigned)e * plane + (unsigned)b * rows + (unsigned)a)); };
+    const int km = clampi(k - 1, g.pges), kp = clampi(k + 1, g.pges);
+    // the fields of `mask` at (i, j, k)
+    auto node = [&](int i, int j, unsigned mask, double v[18]) {
+        const int im = clampi(i - 1, g.rows), ip = clampi(i + 1, g.rows);
+        const int jm = clampi(j - 1, g.cols), jp = clampi(j + 1, g.cols);
+        bool ok = tc.ordinary && ordinary_tool(F(i, j, k)) && ordinary_tool(F(i, jp, k)) && ordinary_tool(F(i, jm, k)) &&
+                  ordinary_tool(F(ip, j, k)) && ordinary_tool(F(im, j, k)) && ordinary_tool(F(i, j, kp)) &&
+                  ordinary_tool(F(i, j, km));
+        if (mask & TOOL_CROSS)
+            ok = ok && ordinary_tool(F(ip, jp, k)) && ordinary_tool(F(im, jm, k)) && ordinary_tool(F(ip, jm, k)) &&
+                 ordinary_tool(F(im, jp, k)) && ordinary_tool(F(ip, j, kp)) && ordinary_tool(F(im, j, km)) &&
+                 ordinary_tool(F(ip, j, km)) && ordinary_tool(F(im, j, kp)) && ordinary_tool(F(i, jp, kp)) &&
+                 ordinary_tool(F(i, jm, km)) && ordinary_tool(F(i, jp, km)) && ordinary_tool(F(i, jm, kp));
+        if (ok)
+            tool64_node<Short64>(F, [&](int a, int b, int e) { return vmax(F(a, b, e), 0.0); }, i, j, k, im, ip, jm, jp,
+                                 km, kp, tc, mask, v);
+        else
+            tool64_general(F, i, j, k, im, ip, jm, jp, km, kp, tc, mask, v);
+    };
+    const int i = i0 + (int)threadIdx.x, j = j0 + (int)threadIdx.y;
+    const bool in = i < g.rows && j < g.cols;
+    double area = 0.0, vol = 0.0;
+    int units = 0;  // volume terms equal to exactly 1
+    // the terms of a node from its Heaviside and Dirac values
+    auto terms = [&](double fc, double heav, double delta) {
+        if (fabs(fc) < thr2ds) area += delta;
+        if (fc < thr2ds) {
+            const double v1 = 1 - heav;  // heav == 0 (no positive neighbour): exactly 1
             if (v1 == 1.0)
-                unit = true;
+                units += 1;
             else
                 vol += v1;
         }
-    }
-    if (o.f[0]) o.f[0][c] = fx;
-    if (o.f[1]) o.f[1][c] = fy;
-    if (o.f[2]) o.f[2][c] = fz;
-    if (o.f[3]) o.f[3][c] = gm;
-    if (o.f[4]) o.f[4][c] = fx / gm;
-    if (o.f[5]) o.f[5][c] = fy / gm;
-    if (o.f[6]) o.f[6][c] = fz / gm;
-    if (o.f[7]) o.f[7][c] = fxx;
-    if (o.f[8]) o.f[8][c] = fyy;
-    if (o.f[9]) o.f[9][c] = fzz;
-    if (o.f[10]) o.f[10][c] = fxy;
-    if (o.f[11]) o.f[11][c] = fyz;
-    if (o.f[12]) o.f[12][c] = fzx;
-    if (o.f[13]) o.f[13][c] = lap;
-    if (o.f[14]) o.f[14][c] = mean;
-    if (o.f[15]) {
-        T q1 = (fyy * fzz - fyz * fyz) * fx + (fzx * fyz - fxy * fzz) * fy + (fxy * fyz - fzx * fyy) * fz;
-        T q2 = (fyz * fzx - fxy * fzz) * fx + (fxx * fzz - fzx * fzx) * fy + (fzx * fxy - fxx * fyz) * fz;
-        T q3 = (fxy * fyz - fyy * fzx) * fx + (fzx * fxy - fxx * fyz) * fy + (fxx * fyy - fxy * fxy) * fz;
-        o.f[15][c] = (fx * q1 + fy * q2 + fz * q3) / gm4;
-    }
-    if (o.f[16]) o.f[16][c] = heav;
-    if (o.f[17]) o.f[17][c] = delta;
-    units += unit ? 1 : 0;
-}
-
-// One node of the toolbox: F(a, b, e) gives the field at row a, column b, page e (clamped
-// coordinates), c the node's offset.  Adds the node's FP64 area and volume terms to area /
-// vol and counts a volume term of exactly 1 in units.
-template <typename T, class Get>
-__device__ __forceinline__ void toolbox_point(Get F, int i, int j, int k, int im, int ip, int jm, int jp, int km,
-                                              int kp, long long c, const ToolboxOut<T> &o, const Grid &g,
-                                              double ds_, T thr2ds, const Recips &rc, double &area, double &vol,
-                                              int &units)
-{
-    static_assert(std::is_same<T, double>::value, "the mixed form's toolbox is k_toolbox_tiled");
-    toolbox_point_f64(F, i, j, k, im, ip, jm, jp, km, kp, c, o, g, ds_, thr2ds, area, vol, units);
-}
-
-// thr2ds: 2 Ds as the smallest T not below it, so that x < thr2ds in T is exactly
-// (double)x < 2 Ds for every x of type T (the reference's FP64 band tests)
-template <typename T>
-__global__ void __launch_bounds__(NT) k_toolbox(const T *__restrict__ f, ToolboxOut<T> o, Grid g, double ds_,
-                                                T thr2ds, double *__restrict__ partials, Recips rc)
-{
-    const int i = blockIdx.x * BX + threadIdx.x;
-    const int j = blockIdx.y * BY + threadIdx.y;
-    const int k = blockIdx.z;
-    double area = 0.0, vol = 0.0;
-    int units = 0;  // volume terms equal to exactly 1
-    if (i < g.rows && j < g.cols) {
+    };
+    const bool direct = want & TOOL_PRIMAL;
+    if (in && want) {
+        double v[18];
+        node(i, j, want, v);
         const long long c = node_index(g, i, j, k);
-        // the clamped neighbour coordinates once; node offsets in 32 bits (grids hold fewer
-        // than 2^31 nodes)
-        const int im = clampi(i - 1, g.rows), ip = clampi(i + 1, g.rows);
-        const int jm = clampi(j - 1, g.cols), jp = clampi(j + 1, g.cols);
-        const int km = clampi(k - 1, g.pges), kp = clampi(k + 1, g.pges);
-        const unsigned rows = (unsigned)g.rows, plane = (unsigned)g.plane;
-        auto F = [&](int a, int b, int e) { return __ldg(f + ((unsigned)e * plane + (unsigned)b * rows + (unsigned)a)); };
-        toolbox_point<T>(F, i, j, k, im, ip, jm, jp, km, kp, c, o, g, ds_, thr2ds, rc, area, vol, units);
+#pragma unroll
+        for (int q = 0; q < 18; ++q)
+            if (o.f[q]) o.f[q][c] = v[q];
+        if (direct) terms(F(i, j, k), v[16], v[17]);
     }
     if (!partials) return;
-    // Volume terms equal to exactly 1 (nodes with no positive neighbour) are counted as
-    // integers; only warps holding other terms run the FP64 shuffle tree.  Per block:
-    // partial = (double)count + FP64 tree sum of the rest, in a fixed order.
+    if (!direct) {
+        __shared__ unsigned count;
+        __shared__ uint8_t list[NT];
+        __shared__ double heav[NT], delta[NT];
+        if (t == 0) count = 0u;
+        __syncthreads();
+        bool need = false;
+        double fc = 0.0;
+        if (in) {
+            fc = F(i, j, k);
+            if (fc < thr2ds) {
+                const double w[7] = {fc,
+                                     F(i, clampi(j + 1, g.cols), k),
+                                     F(i, clampi(j - 1, g.cols), k),
+                                     F(clampi(i + 1, g.rows), j, k),
+                                     F(clampi(i - 1, g.rows), j, k),
+                                     F(i, j, kp),
+                                     F(i, j, km)};
+#pragma unroll
+                for (int q = 0; q < 7; ++q) need = need || w[q] > 0.0 || !ordinary_tool(w[q]);
+                need = need || !tc.ordinary;
+                if (!need) units = 1;
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, need), lane = t & 31;
+        unsigned base = 0;
+        if (m && lane == 0) base = atomicAdd(&count, (unsigned)__popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (need) list[base + __popc(m & ((1u << lane) - 1u))] = (uint8_t)t;
+        __syncthreads();
+        const unsigned n = count;
+        if (t < (int)n) {
+            const int at = list[t];
+            double v[18];
+            node(i0 + at % BX, j0 + at / BX, TOOL_PRIMAL, v);
+            heav[at] = v[16];
+            delta[at] = v[17];
+        }
+        __syncthreads();
+        if (need) terms(fc, heav[t], delta[t]);
+    }
+    // Volume terms equal to exactly 1 are counted as integers; only warps holding other terms run
+    // the FP64 shuffle tree.  Per block: partial = (double)count + FP64 tree sum of the rest, in a
+    // fixed order.
     __shared__ double sa[NW], sv[NW];
     __shared__ int sc[NW];
-    const int t = threadIdx.y * BX + threadIdx.x;
     const int ones = __reduce_add_sync(0xffffffffu, units);
     if (__any_sync(0xffffffffu, area != 0.0)) area = warp_sum(area);
     if (__any_sync(0xffffffffu, vol != 0.0)) vol = warp_sum(vol);
@@ -328,9 +315,9 @@ __global__ void __launch_bounds__(NT) k_toolbox(const T *__restrict__ f, Toolbox
 // which pages k-1, k, k+1 are live while page k+2 is fetched into registers during the
 // page's arithmetic and stored into the slot of page k-2 at its end.  One barrier per
 // page.  Each node is read from memory about once (halo re-reads hit L2), instead of
-// nineteen times through L1 as in k_toolbox.  Per thread the FP64 area and volume terms
-// of its column are summed page by page, then per block in the fixed order of k_toolbox:
-// the same terms as k_toolbox, summed in another fixed order.
+// nineteen times through L1 as in k_toolbox64.  Per thread the FP64 area and volume terms
+// of its column are summed page by page, then per block in the fixed order of k_toolbox64:
+// the same terms, summed in another fixed order.
 constexpr int TB_RING = 4;
 constexpr int TB_SW = BX + 2, TB_SH = BY + 2, TB_PLANE = TB_SW * TB_SH;
 
@@ -525,7 +512,10 @@ cudaError_t launch_toolbox(const T *phi, ToolboxOut<T> out, const Grid &g, doubl
     } else {
         // the plain form: one node per thread, the reference's summation blocks
         if (nblocks) *nblocks = toolbox_partial_blocks(g);
-        k_toolbox<T><<<node_grid(g), dim3(BX, BY), 0, s>>>(phi, out, g, ds, round_up<T>(2 * ds), partials, rc);
+        unsigned want = 0u;
+        for (int q = 0; q < 18; ++q)
+            if (out.f[q]) want |= 1u << q;
+        k_toolbox64<<<node_grid(g), dim3(BX, BY), 0, s>>>(phi, out, g, 2 * ds, partials, tool64(g, ds), want);
     }
     return cudaGetLastError();
 }
