@@ -14,7 +14,10 @@
 #include <cmath>
 #include <limits>
 
+#include <type_traits>
+
 #include "vsl_internal.h"
+#include "vsl_tool64.cuh"
 
 namespace vsl {
 namespace {
@@ -22,16 +25,59 @@ namespace {
 constexpr int ANT = BX * BY;
 constexpr int ANW = ANT / 32;
 
-template <typename T> __device__ __forceinline__ T a_sq(T x) { return x * x; }
-template <typename T> __device__ __forceinline__ T a_cube(T x);
-template <> __device__ __forceinline__ double a_cube<double>(double x) { return pow_cr<3>(x); }
-template <> __device__ __forceinline__ float a_cube<float>(float x) { return x * x * x; }
-template <typename T> __device__ __forceinline__ T a_fourth(T x);
-template <> __device__ __forceinline__ double a_fourth<double>(double x) { return pow_cr<4>(x); }
-template <> __device__ __forceinline__ float a_fourth<float>(float x) { return (x * x) * (x * x); }
+// ---------------------------------------------------------------------------------------
+// Number types of the per-node code.  The plain form takes Short64 (the reference's roundings
+// on the short quotients of vsl_short64.cuh, the FP64 pipe being its bound) where a node's values
+// are ordinary, else double.  The mixed form takes Fast32: quotients as products with the
+// approximate reciprocal, which the compiler shares between equal divisors (a general FP32
+// quotient is about eight instructions, and the kernel issued 900 per node with 60 of them).
+// ---------------------------------------------------------------------------------------
+struct Fast32 {
+    float v;
+    __device__ __forceinline__ Fast32() {}
+    __device__ __forceinline__ Fast32(float x) : v(x) {}
+    friend __device__ __forceinline__ Fast32 operator+(Fast32 a, Fast32 b) { return a.v + b.v; }
+    friend __device__ __forceinline__ Fast32 operator-(Fast32 a, Fast32 b) { return a.v - b.v; }
+    friend __device__ __forceinline__ Fast32 operator-(Fast32 a) { return -a.v; }
+    friend __device__ __forceinline__ Fast32 operator*(Fast32 a, Fast32 b) { return a.v * b.v; }
+    friend __device__ __forceinline__ Fast32 operator/(Fast32 a, Fast32 b) { return a.v * rcp_ftz(b.v); }
+};
+__device__ __forceinline__ float raw64(Fast32 x) { return x.v; }
+struct Divisor32 {
+    float d;
+};
+__device__ __forceinline__ Fast32 operator/(Fast32 a, const Divisor32 &c) { return a.v * rcp_ftz(c.d); }
+template <typename T>
+using AuxDivisors = ToolDivisors<typename std::conditional<std::is_same<T, float>::value, Divisor32, Divisor64>::type>;
+// the mixed form's divisors are products of FP32 spacings
+inline AuxDivisors<float> aux_divisors(const Grid &g, double ds, float)
+{
+    const float x = (float)g.dx, y = (float)g.dy, z = (float)g.dz, s = (float)ds;
+    return AuxDivisors<float>{{{2 * x}, {2 * y}, {2 * z}}, {{x * x}, {y * y}, {z * z}}, {4 * s * s}, true};
+}
+inline AuxDivisors<double> aux_divisors(const Grid &g, double ds, double) { return tool64(g, ds); }
+__device__ __forceinline__ Fast32 a_root(Fast32 x) { return sqrtf(x.v); }
+__device__ __forceinline__ Short64 a_root(Short64 x) { return sqrt(x.v); }
+__device__ __forceinline__ double a_root(double x) { return sqrt(x); }
+template <typename R> __device__ __forceinline__ R a_atleast(R x, R lo)
+{
+    return raw64(x) < raw64(lo) ? lo : x;  // vmax
+}
+// x / g^3, x / g^4 (FP32: general quotients, since the powers leave the normal range where |grad|
+// is near its floor)
+template <typename R> __device__ __forceinline__ R a_over3(R x, R g) { return x / R(pow_cr<3>(raw64(g))); }
+template <> __device__ __forceinline__ Fast32 a_over3(Fast32 x, Fast32 g) { return x.v / (g.v * g.v * g.v); }
+template <typename R> __device__ __forceinline__ R a_over4(R x, R g) { return x / R(pow_cr<4>(raw64(g))); }
+template <> __device__ __forceinline__ Fast32 a_over4(Fast32 x, Fast32 g)
+{
+    return x.v / ((g.v * g.v) * (g.v * g.v));
+}
 
 // the vector norm of shared_utilities.cup:8-12, floored at 1e-14
-template <typename T> __device__ __forceinline__ T a_norm(T x, T y, T z) { return vmax(sqrt(x * x + y * y + z * z), T(1e-14)); }
+template <typename R> __device__ __forceinline__ R a_norm(R x, R y, R z)
+{
+    return a_atleast(a_root(x * x + y * y + z * z), R(1e-14));
+}
 
 __device__ __forceinline__ bool a_node(const Grid &g, int &i, int &j, int &k, long long &c)
 {
@@ -43,36 +89,87 @@ __device__ __forceinline__ bool a_node(const Grid &g, int &i, int &j, int &k, lo
     return true;
 }
 
-// F's toolbox values at one node: gradient, |grad F| (floored), Hessian, normal, and the
-// Heaviside function from the primal max(F, 0) -- tool64_node's expressions in its order
-template <typename T> struct FPart {
-    T fx, fy, fz, gm, nx, ny, nz, fxx, fyy, fzz, fxy, fyz, fzx, heav;
+// offsets of a node's neighbours in 32 bits (grids hold fewer than 2^31 nodes)
+struct Around {
+    int im, ip, jm, jp, km, kp;
+};
+__device__ __forceinline__ Around clamped_around(const Grid &g, int i, int j, int k)
+{
+    const int rows = g.rows, plane = (int)g.plane;
+    return Around{i > 0 ? -1 : 0, i + 1 < g.rows ? 1 : 0, j > 0 ? -rows : 0, j + 1 < g.cols ? rows : 0,
+                  k > 0 ? -plane : 0, k + 1 < g.pges ? plane : 0};
+}
+
+// a field's values around a node: the node, its six neighbours, its twelve edge neighbours
+template <typename T> struct Near {
+    T c, xp, xm, yp, ym, zp, zm, xy[4], yz[4], zx[4];  // (+,+), (-,-), then the two of minus sign
 };
 template <typename T>
-__device__ __forceinline__ FPart<T> f_part(const T *__restrict__ f, const Grid &g, int i, int j, int k, long long c,
-                                           T dx, T dy, T dz, T ds)
+__device__ __forceinline__ Near<T> load_near(const T *__restrict__ f, long long c, const Around &n, bool cross)
 {
-    auto F = [&](int a, int b, int e) { return __ldg(f + clamped_index(g, a, b, e)); };
-    FPart<T> r;
-    const T fc = __ldg(f + c);
-    const T fxp = F(i, j + 1, k), fxm = F(i, j - 1, k), fyp = F(i + 1, j, k), fym = F(i - 1, j, k);
-    const T fzp = F(i, j, k + 1), fzm = F(i, j, k - 1);
-    r.fx = (fxp - fxm) / (2 * dx);
-    r.fy = (fyp - fym) / (2 * dy);
-    r.fz = (fzp - fzm) / (2 * dz);
-    r.gm = vmax(sqrt(r.fx * r.fx + r.fy * r.fy + r.fz * r.fz), T(1e-14));
+    const T *p = f + c;
+    auto at = [&](int o) { return __ldg(p + o); };
+    Near<T> r;
+    r.c = at(0);
+    r.xp = at(n.jp);
+    r.xm = at(n.jm);
+    r.yp = at(n.ip);
+    r.ym = at(n.im);
+    r.zp = at(n.kp);
+    r.zm = at(n.km);
+    if (cross) {
+        r.xy[0] = at(n.ip + n.jp);
+        r.xy[1] = at(n.im + n.jm);
+        r.xy[2] = at(n.ip + n.jm);
+        r.xy[3] = at(n.im + n.jp);
+        r.yz[0] = at(n.ip + n.kp);
+        r.yz[1] = at(n.im + n.km);
+        r.yz[2] = at(n.ip + n.km);
+        r.yz[3] = at(n.im + n.kp);
+        r.zx[0] = at(n.jp + n.kp);
+        r.zx[1] = at(n.jm + n.km);
+        r.zx[2] = at(n.jp + n.km);
+        r.zx[3] = at(n.jm + n.kp);
+    }
+    return r;
+}
+__device__ __forceinline__ bool ordinary_near(const Near<double> &r, bool cross)
+{
+    bool ok = ordinary_tool(r.c) && ordinary_tool(r.xp) && ordinary_tool(r.xm) && ordinary_tool(r.yp) &&
+              ordinary_tool(r.ym) && ordinary_tool(r.zp) && ordinary_tool(r.zm);
+    if (cross)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ok = ok && ordinary_tool(r.xy[q]) && ordinary_tool(r.yz[q]) && ordinary_tool(r.zx[q]);
+    return ok;
+}
+
+// F's toolbox values at one node: gradient, |grad F| (floored), Hessian, normal, and the
+// Heaviside function from the primal max(F, 0) -- tool64_node's expressions in its order
+template <typename R> struct FPart {
+    R fx, fy, fz, gm, nx, ny, nz, fxx, fyy, fzz, fxy, fyz, fzx, heav;
+};
+template <typename R, typename T>
+__device__ __forceinline__ FPart<R> f_part(const Near<T> &f, const AuxDivisors<T> &t)
+{
+    FPart<R> r;
+    auto pos = [](T x) { return R(vmax(x, T(0))); };
+    r.fx = (R(f.xp) - R(f.xm)) / t.two[0];
+    r.fy = (R(f.yp) - R(f.ym)) / t.two[1];
+    r.fz = (R(f.zp) - R(f.zm)) / t.two[2];
+    r.gm = a_norm(r.fx, r.fy, r.fz);
     r.nx = r.fx / r.gm;
     r.ny = r.fy / r.gm;
     r.nz = r.fz / r.gm;
-    r.fxx = (fxp - 2 * fc + fxm) / (dx * dx);
-    r.fyy = (fyp - 2 * fc + fym) / (dy * dy);
-    r.fzz = (fzp - 2 * fc + fzm) / (dz * dz);
-    r.fxy = (F(i + 1, j + 1, k) + F(i - 1, j - 1, k) - F(i + 1, j - 1, k) - F(i - 1, j + 1, k)) / (4 * ds * ds);
-    r.fyz = (F(i + 1, j, k + 1) + F(i - 1, j, k - 1) - F(i + 1, j, k - 1) - F(i - 1, j, k + 1)) / (4 * ds * ds);
-    r.fzx = (F(i, j + 1, k + 1) + F(i, j - 1, k - 1) - F(i, j + 1, k - 1) - F(i, j - 1, k + 1)) / (4 * ds * ds);
-    const T px = (vmax(fxp, T(0)) - vmax(fxm, T(0))) / (2 * dx);
-    const T py = (vmax(fyp, T(0)) - vmax(fym, T(0))) / (2 * dy);
-    const T pz = (vmax(fzp, T(0)) - vmax(fzm, T(0))) / (2 * dz);
+    const R two(2), c(f.c);
+    r.fxx = (R(f.xp) - two * c + R(f.xm)) / t.sq[0];
+    r.fyy = (R(f.yp) - two * c + R(f.ym)) / t.sq[1];
+    r.fzz = (R(f.zp) - two * c + R(f.zm)) / t.sq[2];
+    r.fxy = (R(f.xy[0]) + R(f.xy[1]) - R(f.xy[2]) - R(f.xy[3])) / t.four;
+    r.fyz = (R(f.yz[0]) + R(f.yz[1]) - R(f.yz[2]) - R(f.yz[3])) / t.four;
+    r.fzx = (R(f.zx[0]) + R(f.zx[1]) - R(f.zx[2]) - R(f.zx[3])) / t.four;
+    const R px = (pos(f.xp) - pos(f.xm)) / t.two[0];
+    const R py = (pos(f.yp) - pos(f.ym)) / t.two[1];
+    const R pz = (pos(f.zp) - pos(f.zm)) / t.two[2];
     r.heav = (px * r.fx + py * r.fy + pz * r.fz) / (r.gm * r.gm);
     return r;
 }
@@ -84,205 +181,261 @@ enum AuxField {
     AU_AHEAV, AU_ADELTA, AU_KERNEL_FIELDS
 };
 
-// auxi_set_calculus_toolbox.cu:27-197 at node (i,j,k): A's central differences (clamped,
-// `Aat`), the primal of its Heaviside (`Pat`), F's values at the node given.
-template <typename T, class AFn, class PFn>
-__device__ __forceinline__ void aux_core(AFn Aat, PFn Pat, const FPart<T> &fp, int i, int j, int k, T dx, T dy, T dz,
-                                         T ds, T v[AU_KERNEL_FIELDS])
+// auxi_set_calculus_toolbox.cu:27-197 at one node: A's values `a`, its primal's `p` (the node and
+// its six neighbours), F's toolbox values.
+template <typename R, typename T>
+__device__ __forceinline__ void aux_core(const Near<T> &a, const Near<T> &p, const FPart<R> &fp, const AuxDivisors<T> &t,
+                                         T v[AU_KERNEL_FIELDS])
 {
-    const T ac = Aat(i, j, k);
-    const T axp = Aat(i, j + 1, k), axm = Aat(i, j - 1, k), ayp = Aat(i + 1, j, k), aym = Aat(i - 1, j, k);
-    const T azp = Aat(i, j, k + 1), azm = Aat(i, j, k - 1);
-    const T ax = (axp - axm) / (2 * dx);
-    const T ay = (ayp - aym) / (2 * dy);
-    const T az = (azp - azm) / (2 * dz);
-    const T agm = a_norm(ax, ay, az);
-    v[AU_AX] = ax;
-    v[AU_AY] = ay;
-    v[AU_AZ] = az;
-    v[AU_AGRADMAG] = agm;
-    const T fx = fp.fx, fy = fp.fy, fz = fp.fz;
-    const T cx = fy * az - fz * ay, cy = fz * ax - fx * az, cz = fx * ay - fy * ax;
-    const T ncr = a_norm(cx, cy, cz);
-    v[AU_CX] = cx;
-    v[AU_CY] = cy;
-    v[AU_CZ] = cz;
-    v[AU_NORMCROSS] = ncr;
-    const T tx = cx / ncr, ty = cy / ncr, tz = cz / ncr;
-    v[AU_TX] = tx;
-    v[AU_TY] = ty;
-    v[AU_TZ] = tz;
-    const T nx = ty * fp.nz - tz * fp.ny, ny = tz * fp.nx - tx * fp.nz, nz = tx * fp.ny - ty * fp.nx;
-    v[AU_NX] = nx;
-    v[AU_NY] = ny;
-    v[AU_NZ] = nz;
-    const T axx = (axp - 2 * ac + axm) / (dx * dx);
-    const T ayy = (ayp - 2 * ac + aym) / (dy * dy);
-    const T azz = (azp - 2 * ac + azm) / (dz * dz);
-    const T axy = (Aat(i + 1, j + 1, k) + Aat(i - 1, j - 1, k) - Aat(i + 1, j - 1, k) - Aat(i - 1, j + 1, k)) / (4 * ds * ds);
-    const T ayz = (Aat(i + 1, j, k + 1) + Aat(i - 1, j, k - 1) - Aat(i + 1, j, k - 1) - Aat(i - 1, j, k + 1)) / (4 * ds * ds);
-    const T azx = (Aat(i, j + 1, k + 1) + Aat(i, j - 1, k - 1) - Aat(i, j + 1, k - 1) - Aat(i, j - 1, k + 1)) / (4 * ds * ds);
-    const T alap = axx + ayy + azz;
-    v[AU_AXX] = axx;
-    v[AU_AYY] = ayy;
-    v[AU_AZZ] = azz;
-    v[AU_AXY] = axy;
-    v[AU_AYZ] = ayz;
-    v[AU_AZX] = azx;
-    v[AU_ALAP] = alap;
-    const T fxx = fp.fxx, fyy = fp.fyy, fzz = fp.fzz, fxy = fp.fxy, fyz = fp.fyz, fzx = fp.fzx, fgm = fp.gm;
+    const R ax = (R(a.xp) - R(a.xm)) / t.two[0];
+    const R ay = (R(a.yp) - R(a.ym)) / t.two[1];
+    const R az = (R(a.zp) - R(a.zm)) / t.two[2];
+    const R agm = a_norm(ax, ay, az);
+    v[AU_AX] = raw64(ax);
+    v[AU_AY] = raw64(ay);
+    v[AU_AZ] = raw64(az);
+    v[AU_AGRADMAG] = raw64(agm);
+    const R fx = fp.fx, fy = fp.fy, fz = fp.fz;
+    const R cx = fy * az - fz * ay, cy = fz * ax - fx * az, cz = fx * ay - fy * ax;
+    const R ncr = a_norm(cx, cy, cz);
+    v[AU_CX] = raw64(cx);
+    v[AU_CY] = raw64(cy);
+    v[AU_CZ] = raw64(cz);
+    v[AU_NORMCROSS] = raw64(ncr);
+    const R tx = cx / ncr, ty = cy / ncr, tz = cz / ncr;
+    v[AU_TX] = raw64(tx);
+    v[AU_TY] = raw64(ty);
+    v[AU_TZ] = raw64(tz);
+    const R nx = ty * fp.nz - tz * fp.ny, ny = tz * fp.nx - tx * fp.nz, nz = tx * fp.ny - ty * fp.nx;
+    v[AU_NX] = raw64(nx);
+    v[AU_NY] = raw64(ny);
+    v[AU_NZ] = raw64(nz);
+    const R two(2), ac(a.c);
+    const R axx = (R(a.xp) - two * ac + R(a.xm)) / t.sq[0];
+    const R ayy = (R(a.yp) - two * ac + R(a.ym)) / t.sq[1];
+    const R azz = (R(a.zp) - two * ac + R(a.zm)) / t.sq[2];
+    const R axy = (R(a.xy[0]) + R(a.xy[1]) - R(a.xy[2]) - R(a.xy[3])) / t.four;
+    const R ayz = (R(a.yz[0]) + R(a.yz[1]) - R(a.yz[2]) - R(a.yz[3])) / t.four;
+    const R azx = (R(a.zx[0]) + R(a.zx[1]) - R(a.zx[2]) - R(a.zx[3])) / t.four;
+    const R alap = axx + ayy + azz;
+    v[AU_AXX] = raw64(axx);
+    v[AU_AYY] = raw64(ayy);
+    v[AU_AZZ] = raw64(azz);
+    v[AU_AXY] = raw64(axy);
+    v[AU_AYZ] = raw64(ayz);
+    v[AU_AZX] = raw64(azx);
+    v[AU_ALAP] = raw64(alap);
+    const R fxx = fp.fxx, fyy = fp.fyy, fzz = fp.fzz, fxy = fp.fxy, fyz = fp.fyz, fzx = fp.fzx, fgm = fp.gm;
     // geodesic curvature n . ((H_F t) x grad A + grad F x (H_A t)) / |grad F x grad A|
-    T vx = tx * fxx + ty * fxy + tz * fzx;
-    T vy = tx * fxy + ty * fyy + tz * fyz;
-    T vz = tx * fzx + ty * fyz + tz * fzz;
-    const T w1x = vy * az - vz * ay, w1y = vz * ax - vx * az, w1z = vx * ay - vy * ax;
+    R vx = tx * fxx + ty * fxy + tz * fzx;
+    R vy = tx * fxy + ty * fyy + tz * fyz;
+    R vz = tx * fzx + ty * fyz + tz * fzz;
+    const R w1x = vy * az - vz * ay, w1y = vz * ax - vx * az, w1z = vx * ay - vy * ax;
     vx = tx * axx + ty * axy + tz * azx;
     vy = tx * axy + ty * ayy + tz * ayz;
     vz = tx * azx + ty * ayz + tz * azz;
-    const T w2x = fy * vz - fz * vy, w2y = fz * vx - fx * vz, w2z = fx * vy - fy * vx;
-    v[AU_GEODESIC] = (nx * (w1x + w2x) + ny * (w1y + w2y) + nz * (w1z + w2z)) / ncr;
+    const R w2x = fy * vz - fz * vy, w2y = fz * vx - fx * vz, w2z = fx * vy - fy * vx;
+    v[AU_GEODESIC] = raw64((nx * (w1x + w2x) + ny * (w1y + w2y) + nz * (w1z + w2z)) / ncr);
     // grad N = H_F / |grad F| - grad F (H_F grad F)^T / |grad F|^3
-    const T g3 = a_cube(fgm);
-    const T r1 = fxx * fx + fxy * fy + fzx * fz;
-    const T r2 = fxy * fx + fyy * fy + fyz * fz;
-    const T r3 = fzx * fx + fyz * fy + fzz * fz;
-    const T Nxx = fxx / fgm - fx * r1 / g3, Nyx = fxy / fgm - fy * r1 / g3, Nzx = fzx / fgm - fz * r1 / g3;
-    const T Nxy = fxy / fgm - fx * r2 / g3, Nyy = fyy / fgm - fy * r2 / g3, Nzy = fyz / fgm - fz * r2 / g3;
-    const T Nxz = fzx / fgm - fx * r3 / g3, Nyz = fyz / fgm - fy * r3 / g3, Nzz = fzz / fgm - fz * r3 / g3;
+    const R r1 = fxx * fx + fxy * fy + fzx * fz;
+    const R r2 = fxy * fx + fyy * fy + fyz * fz;
+    const R r3 = fzx * fx + fyz * fy + fzz * fz;
+    const R Nxx = fxx / fgm - a_over3(fx * r1, fgm), Nyx = fxy / fgm - a_over3(fy * r1, fgm),
+            Nzx = fzx / fgm - a_over3(fz * r1, fgm);
+    const R Nxy = fxy / fgm - a_over3(fx * r2, fgm), Nyy = fyy / fgm - a_over3(fy * r2, fgm),
+            Nzy = fyz / fgm - a_over3(fz * r2, fgm);
+    const R Nxz = fzx / fgm - a_over3(fx * r3, fgm), Nyz = fyz / fgm - a_over3(fy * r3, fgm),
+            Nzz = fzz / fgm - a_over3(fz * r3, fgm);
     vx = Nxx * tx + Nxy * ty + Nxz * tz;
     vy = Nyx * tx + Nyy * ty + Nyz * tz;
     vz = Nzx * tx + Nzy * ty + Nzz * tz;
-    v[AU_NORMALCURV] = -(tx * vx + ty * vy + tz * vz);
+    v[AU_NORMALCURV] = raw64(-(tx * vx + ty * vy + tz * vz));
     vx = Nxx * nx + Nxy * ny + Nxz * nz;
     vy = Nyx * nx + Nyy * ny + Nyz * nz;
     vz = Nzx * nx + Nzy * ny + Nzz * nz;
-    v[AU_TORSION] = -(tx * vx + ty * vy + tz * vz);
-    v[AU_BPERP] = -(nx * vx + ny * vy + nz * vz);
+    v[AU_TORSION] = raw64(-(tx * vx + ty * vy + tz * vz));
+    v[AU_BPERP] = raw64(-(nx * vx + ny * vy + nz * vz));
     // Heaviside and Dirac functions of A from its primal
-    const T pc = Pat(i, j, k);
-    const T pxp = Pat(i, j + 1, k), pxm = Pat(i, j - 1, k), pyp = Pat(i + 1, j, k), pym = Pat(i - 1, j, k);
-    const T pzp = Pat(i, j, k + 1), pzm = Pat(i, j, k - 1);
-    const T px = (pxp - pxm) / (2 * dx), py = (pyp - pym) / (2 * dy), pz = (pzp - pzm) / (2 * dz);
-    const T dot = px * ax + py * ay + pz * az;
-    v[AU_AHEAV] = dot / a_sq(agm);
-    const T pxx = (pxp - 2 * pc + pxm) / (dx * dx);
-    const T pyy = (pyp - 2 * pc + pym) / (dy * dy);
-    const T pzz = (pzp - 2 * pc + pzm) / (dz * dz);
-    const T plap = pxx + pyy + pzz;
-    v[AU_ADELTA] = plap / a_sq(agm) - dot * alap / a_fourth(agm);
+    const R px = (R(p.xp) - R(p.xm)) / t.two[0], py = (R(p.yp) - R(p.ym)) / t.two[1],
+            pz = (R(p.zp) - R(p.zm)) / t.two[2];
+    const R dot = px * ax + py * ay + pz * az;
+    const R pc(p.c);
+    v[AU_AHEAV] = raw64(dot / (agm * agm));
+    const R pxx = (R(p.xp) - two * pc + R(p.xm)) / t.sq[0];
+    const R pyy = (R(p.yp) - two * pc + R(p.ym)) / t.sq[1];
+    const R pzz = (R(p.zp) - two * pc + R(p.zm)) / t.sq[2];
+    const R plap = pxx + pyy + pzz;
+    v[AU_ADELTA] = raw64(plap / (agm * agm) - a_over4(dot * alap, agm));
 }
 
 // the reference kernel's own form: F's toolbox fields and AHPrimal read from arrays
-template <typename T>
-__global__ void __launch_bounds__(ANT) k_auxi_dropin(AuxOut<T> o, const T *__restrict__ lsf,
-                                                     const T *__restrict__ ahp, AuxFIn<T> fin, Grid g, T ds)
+template <typename R>
+__device__ __forceinline__ void auxi_dropin_node(const Near<double> &a, const Near<double> &p, const double fin[13],
+                                                 const Tool64 &t, double v[AU_KERNEL_FIELDS])
+{
+    FPart<R> fp;
+    fp.fx = R(fin[0]);
+    fp.fy = R(fin[1]);
+    fp.fz = R(fin[2]);
+    fp.gm = R(fin[3]);
+    fp.nx = R(fin[4]);
+    fp.ny = R(fin[5]);
+    fp.nz = R(fin[6]);
+    fp.fxx = R(fin[7]);
+    fp.fyy = R(fin[8]);
+    fp.fzz = R(fin[9]);
+    fp.fxy = R(fin[10]);
+    fp.fyz = R(fin[11]);
+    fp.fzx = R(fin[12]);
+    aux_core<R>(a, p, fp, t, v);
+}
+__global__ void __launch_bounds__(ANT) k_auxi_dropin(const __grid_constant__ AuxOut<double> o,
+                                                     const double *__restrict__ lsf, const double *__restrict__ ahp,
+                                                     const __grid_constant__ AuxFIn<double> fin,
+                                                     const __grid_constant__ Grid g, const __grid_constant__ Tool64 t)
 {
     int i, j, k;
     long long c;
     if (!a_node(g, i, j, k, c)) return;
-    const T dx = (T)g.dx, dy = (T)g.dy, dz = (T)g.dz;
-    FPart<T> fp;
-    fp.fx = fin.f[0][c];
-    fp.fy = fin.f[1][c];
-    fp.fz = fin.f[2][c];
-    fp.gm = fin.f[3][c];
-    fp.nx = fin.f[4][c];
-    fp.ny = fin.f[5][c];
-    fp.nz = fin.f[6][c];
-    fp.fxx = fin.f[7][c];
-    fp.fyy = fin.f[8][c];
-    fp.fzz = fin.f[9][c];
-    fp.fxy = fin.f[10][c];
-    fp.fyz = fin.f[11][c];
-    fp.fzx = fin.f[12][c];
-    T v[AU_KERNEL_FIELDS];
-    aux_core<T>([&](int a, int b, int e) { return __ldg(lsf + clamped_index(g, a, b, e)); },
-                [&](int a, int b, int e) { return __ldg(ahp + clamped_index(g, a, b, e)); }, fp, i, j, k, dx, dy, dz,
-                ds, v);
+    const Around n = clamped_around(g, i, j, k);
+    const Near<double> a = load_near(lsf, c, n, true), p = load_near(ahp, c, n, false);
+    double f[13], v[AU_KERNEL_FIELDS];
+    // the caller's F fields are divided by too: |grad F| a normal divisor, the others as the values
+    bool ok = t.ordinary && ordinary_near(a, true) && ordinary_near(p, false);
+#pragma unroll
+    for (int q = 0; q < 13; ++q) {
+        f[q] = fin.f[q][c];
+        ok = ok && ordinary_tool(f[q]);
+    }
+    ok = ok && f[3] >= 1e-14;
+    if (ok)
+        auxi_dropin_node<Short64>(a, p, f, t, v);
+    else
+        auxi_dropin_node<double>(a, p, f, t, v);
 #pragma unroll
     for (int q = 0; q < AU_KERNEL_FIELDS; ++q) o.f[q][c] = v[q];
 }
 
 // pass 1 of the fused form: F recomputed, AHPrimal = max(A, 0) on the fly; writes the
-// requested fields, and the values pass 2 needs into `keep` (outputs or workspace):
-// C, |C|, |grad A|, ADiracDelta, AHeaviside and F's Heaviside
+// requested fields, and the values pass 2 needs into `keep` where they are not requested
+// (null: not needed): C, |C|, |grad A|, ADiracDelta, AHeaviside and F's Heaviside
+template <typename R, typename T>
+__device__ __forceinline__ void aux_node(const Near<T> &a, const Near<T> &f, const AuxDivisors<T> &t, T v[AU_KERNEL_FIELDS],
+                                         T &fheav)
+{
+    const FPart<R> fp = f_part<R>(f, t);
+    Near<T> p;
+    auto pos = [](T x) { return vmax(x, T(0)); };
+    p.c = pos(a.c);
+    p.xp = pos(a.xp);
+    p.xm = pos(a.xm);
+    p.yp = pos(a.yp);
+    p.ym = pos(a.ym);
+    p.zp = pos(a.zp);
+    p.zm = pos(a.zm);
+    aux_core<R>(a, p, fp, t, v);
+    fheav = raw64(fp.heav);
+}
 template <typename T>
-__global__ void __launch_bounds__(ANT) k_aux_pass1(const T *__restrict__ A, const T *__restrict__ F, AuxOut<T> o,
-                                                   AuxKeep<T> keep, Grid g, T ds)
+__global__ void __launch_bounds__(ANT) k_aux_pass1(const T *__restrict__ A, const T *__restrict__ F,
+                                                   const __grid_constant__ AuxOut<T> o,
+                                                   const __grid_constant__ AuxKeep<T> keep,
+                                                   const __grid_constant__ Grid g, const __grid_constant__ AuxDivisors<T> t)
 {
     int i, j, k;
     long long c;
     if (!a_node(g, i, j, k, c)) return;
-    const T dx = (T)g.dx, dy = (T)g.dy, dz = (T)g.dz;
-    const FPart<T> fp = f_part(F, g, i, j, k, c, dx, dy, dz, ds);
-    T v[AU_KERNEL_FIELDS];
-    aux_core<T>([&](int a, int b, int e) { return __ldg(A + clamped_index(g, a, b, e)); },
-                [&](int a, int b, int e) { return vmax(__ldg(A + clamped_index(g, a, b, e)), T(0)); }, fp, i, j, k,
-                dx, dy, dz, ds, v);
+    const Around n = clamped_around(g, i, j, k);
+    const Near<T> a = load_near(A, c, n, true), f = load_near(F, c, n, true);
+    T v[AU_KERNEL_FIELDS], fheav;
+    if constexpr (std::is_same<T, float>::value) {
+        aux_node<Fast32>(a, f, t, v, fheav);
+    } else {
+        if (t.ordinary && ordinary_near(a, true) && ordinary_near(f, true))
+            aux_node<Short64>(a, f, t, v, fheav);
+        else
+            aux_node<double>(a, f, t, v, fheav);
+    }
 #pragma unroll
     for (int q = 0; q < AU_KERNEL_FIELDS; ++q)
         if (o.f[q]) o.f[q][c] = v[q];
-    keep.cx[c] = v[AU_CX];
-    keep.cy[c] = v[AU_CY];
-    keep.cz[c] = v[AU_CZ];
-    keep.ncr[c] = v[AU_NORMCROSS];
-    keep.agm[c] = v[AU_AGRADMAG];
-    keep.adelta[c] = v[AU_ADELTA];
-    keep.aheav[c] = v[AU_AHEAV];
-    keep.fheav[c] = fp.heav;
+    if (keep.cx) keep.cx[c] = v[AU_CX];
+    if (keep.cy) keep.cy[c] = v[AU_CY];
+    if (keep.cz) keep.cz[c] = v[AU_CZ];
+    if (keep.ncr) keep.ncr[c] = v[AU_NORMCROSS];
+    if (keep.agm) keep.agm[c] = v[AU_AGRADMAG];
+    if (keep.adelta) keep.adelta[c] = v[AU_ADELTA];
+    if (keep.aheav) keep.aheav[c] = v[AU_AHEAV];
+    if (keep.fheav) keep.fheav[c] = fheav;
 }
 
 // periodic neighbours of SD.GD3 (circshift)
-struct PNb {
-    int ip, im, jp, jm, kp, km;
-};
-__device__ __forceinline__ PNb periodic_nb(const Grid &g, int i, int j, int k)
+__device__ __forceinline__ Around periodic_around(const Grid &g, int i, int j, int k)
 {
-    PNb n;
-    n.jp = j + 1 == g.cols ? 0 : j + 1;
-    n.jm = j == 0 ? g.cols - 1 : j - 1;
-    n.ip = i + 1 == g.rows ? 0 : i + 1;
-    n.im = i == 0 ? g.rows - 1 : i - 1;
-    n.kp = k + 1 == g.pges ? 0 : k + 1;
-    n.km = k == 0 ? g.pges - 1 : k - 1;
-    return n;
+    const int rows = g.rows, plane = (int)g.plane;
+    return Around{i > 0 ? -1 : g.rows - 1,          i + 1 < g.rows ? 1 : 1 - g.rows,
+                  j > 0 ? -rows : (g.cols - 1) * rows, j + 1 < g.cols ? rows : (1 - g.cols) * rows,
+                  k > 0 ? -plane : (g.pges - 1) * plane, k + 1 < g.pges ? plane : (1 - g.pges) * plane};
 }
 
 // pass 2: AFDiracDelta = (C . (grad H_F x grad H_A)) / |C|^2 with GD3.Gradient, and
 // ADiracDeltaDn = (Laplacian(H_A) - ADiracDelta Laplacian(A)) / |grad A| with GD3.Laplacian
 // (GPUAsetCalculusToolBox.m:56-61)
+template <typename R, typename T>
+__device__ __forceinline__ T aux_afd(const Near<T> &h1, const Near<T> &h2, T cx, T cy, T cz, T ncr, const AuxDivisors<T> &t)
+{
+    const R h1x = (R(h1.xp) - R(h1.xm)) / t.two[0], h1y = (R(h1.yp) - R(h1.ym)) / t.two[1],
+            h1z = (R(h1.zp) - R(h1.zm)) / t.two[2];
+    const R h2x = (R(h2.xp) - R(h2.xm)) / t.two[0], h2y = (R(h2.yp) - R(h2.ym)) / t.two[1],
+            h2z = (R(h2.zp) - R(h2.zm)) / t.two[2];
+    const R chx = h2y * h1z - h2z * h1y, chy = h2z * h1x - h2x * h1z, chz = h2x * h1y - h2y * h1x;
+    const R dot = R(cx) * chx + R(cy) * chy + R(cz) * chz;
+    return raw64(dot / (R(ncr) * R(ncr)));
+}
+template <typename R, typename T> __device__ __forceinline__ R aux_lap(const Near<T> &f, const AuxDivisors<T> &t)
+{
+    const R two(2), c(f.c);
+    const R fxx = (R(f.xp) - two * c + R(f.xm)) / t.sq[0];
+    const R fyy = (R(f.yp) - two * c + R(f.ym)) / t.sq[1];
+    const R fzz = (R(f.zp) - two * c + R(f.zm)) / t.sq[2];
+    return fxx + fyy + fzz;
+}
+template <typename R, typename T>
+__device__ __forceinline__ T aux_ddn(const Near<T> &h, const Near<T> &a, T adelta, T agm, const AuxDivisors<T> &t)
+{
+    return raw64((aux_lap<R>(h, t) - R(adelta) * aux_lap<R>(a, t)) / R(agm));
+}
 template <typename T>
-__global__ void __launch_bounds__(ANT) k_aux_pass2(const T *__restrict__ A, AuxKeepC<T> keep, T *__restrict__ afd,
-                                                   T *__restrict__ addn, Grid g)
+__global__ void __launch_bounds__(ANT) k_aux_pass2(const T *__restrict__ A, const __grid_constant__ AuxKeepC<T> keep,
+                                                   T *__restrict__ afd, T *__restrict__ addn,
+                                                   const __grid_constant__ Grid g, const __grid_constant__ AuxDivisors<T> t)
 {
     int i, j, k;
     long long c;
     if (!a_node(g, i, j, k, c)) return;
-    const T dx = (T)g.dx, dy = (T)g.dy, dz = (T)g.dz;
-    const PNb n = periodic_nb(g, i, j, k);
-    auto at = [&](const T *f, int a, int b, int e) { return __ldg(f + node_index(g, a, b, e)); };
+    const Around n = periodic_around(g, i, j, k);
+    const Near<T> h1 = load_near(keep.aheav, c, n, false);
     if (afd) {
-        const T *h1 = keep.aheav, *h2 = keep.fheav;
-        const T h1x = (at(h1, i, n.jp, k) - at(h1, i, n.jm, k)) / (2 * dx);
-        const T h1y = (at(h1, n.ip, j, k) - at(h1, n.im, j, k)) / (2 * dy);
-        const T h1z = (at(h1, i, j, n.kp) - at(h1, i, j, n.km)) / (2 * dz);
-        const T h2x = (at(h2, i, n.jp, k) - at(h2, i, n.jm, k)) / (2 * dx);
-        const T h2y = (at(h2, n.ip, j, k) - at(h2, n.im, j, k)) / (2 * dy);
-        const T h2z = (at(h2, i, j, n.kp) - at(h2, i, j, n.km)) / (2 * dz);
-        const T chx = h2y * h1z - h2z * h1y, chy = h2z * h1x - h2x * h1z, chz = h2x * h1y - h2y * h1x;
-        const T dot = __ldg(keep.cx + c) * chx + __ldg(keep.cy + c) * chy + __ldg(keep.cz + c) * chz;
-        const T ncr = __ldg(keep.ncr + c);
-        afd[c] = dot / (ncr * ncr);
+        const Near<T> h2 = load_near(keep.fheav, c, n, false);
+        const T cx = __ldg(keep.cx + c), cy = __ldg(keep.cy + c), cz = __ldg(keep.cz + c), ncr = __ldg(keep.ncr + c);
+        if constexpr (std::is_same<T, float>::value)
+            afd[c] = aux_afd<Fast32>(h1, h2, cx, cy, cz, ncr, t);
+        else if (t.ordinary && ordinary_near(h1, false) && ordinary_near(h2, false) && ordinary_tool(cx) &&
+                 ordinary_tool(cy) && ordinary_tool(cz) && ordinary_tool(ncr))
+            afd[c] = aux_afd<Short64>(h1, h2, cx, cy, cz, ncr, t);
+        else
+            afd[c] = aux_afd<double>(h1, h2, cx, cy, cz, ncr, t);
     }
     if (addn) {
-        auto lap = [&](const T *f) {
-            const T fc = __ldg(f + c);
-            const T fxx = (at(f, i, n.jp, k) - T(2) * fc + at(f, i, n.jm, k)) / (dx * dx);
-            const T fyy = (at(f, n.ip, j, k) - T(2) * fc + at(f, n.im, j, k)) / (dy * dy);
-            const T fzz = (at(f, i, j, n.kp) - T(2) * fc + at(f, i, j, n.km)) / (dz * dz);
-            return fxx + fyy + fzz;
-        };
-        addn[c] = (lap(keep.aheav) - __ldg(keep.adelta + c) * lap(A)) / __ldg(keep.agm + c);
+        const Near<T> a = load_near(A, c, n, false);
+        const T adelta = __ldg(keep.adelta + c), agm = __ldg(keep.agm + c);
+        if constexpr (std::is_same<T, float>::value)
+            addn[c] = aux_ddn<Fast32>(h1, a, adelta, agm, t);
+        else if (t.ordinary && ordinary_near(h1, false) && ordinary_near(a, false) && ordinary_tool(adelta) &&
+                 ordinary_tool(agm))
+            addn[c] = aux_ddn<Short64>(h1, a, adelta, agm, t);
+        else
+            addn[c] = aux_ddn<double>(h1, a, adelta, agm, t);
     }
 }
 
@@ -334,13 +487,32 @@ cudaError_t launch_aux_toolbox(const T *A, const T *F, AuxOut<T> o, AuxKeep<T> k
                                cudaStream_t s)
 {
     const dim3 gr = node_grid(g), bl(BX, BY);
-    k_aux_pass1<T><<<gr, bl, 0, s>>>(A, F, o, keep, g, (T)ds);
+    const AuxDivisors<T> t = aux_divisors(g, ds, T(0));
+    T *afd = o.f[AU_KERNEL_FIELDS], *addn = o.f[AU_KERNEL_FIELDS + 1];
+    // pass 2 reads the caller's arrays where the caller asked for those fields; pass 1 stores in
+    // `keep` what pass 2 needs of the others
+    AuxKeepC<T> kc{keep.cx, keep.cy, keep.cz, keep.ncr, keep.agm, keep.adelta, keep.aheav, keep.fheav};
+    auto from = [&](T *&k, const T *&r, int field, bool needed) {
+        if (!needed) {
+            k = nullptr;
+        } else if (o.f[field]) {
+            r = o.f[field];
+            k = nullptr;
+        }
+    };
+    from(keep.cx, kc.cx, AU_CX, afd);
+    from(keep.cy, kc.cy, AU_CY, afd);
+    from(keep.cz, kc.cz, AU_CZ, afd);
+    from(keep.ncr, kc.ncr, AU_NORMCROSS, afd);
+    from(keep.agm, kc.agm, AU_AGRADMAG, addn);
+    from(keep.adelta, kc.adelta, AU_ADELTA, addn);
+    from(keep.aheav, kc.aheav, AU_AHEAV, afd || addn);
+    if (!afd) keep.fheav = nullptr;
+    k_aux_pass1<T><<<gr, bl, 0, s>>>(A, F, o, keep, g, t);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    T *afd = o.f[AU_KERNEL_FIELDS], *addn = o.f[AU_KERNEL_FIELDS + 1];
     if (!afd && !addn) return cudaSuccess;
-    AuxKeepC<T> kc{keep.cx, keep.cy, keep.cz, keep.ncr, keep.agm, keep.adelta, keep.aheav, keep.fheav};
-    k_aux_pass2<T><<<gr, bl, 0, s>>>(A, kc, afd, addn, g);
+    k_aux_pass2<T><<<gr, bl, 0, s>>>(A, kc, afd, addn, g, t);
     return cudaGetLastError();
 }
 

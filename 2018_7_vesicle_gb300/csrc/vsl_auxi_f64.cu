@@ -10,7 +10,7 @@ VSL_INSTANTIATE_AUXI(double)
 cudaError_t launch_auxi_dropin(AuxOut<double> o, const double *lsf, const double *ahp, AuxFIn<double> fin,
                                const Grid &g, double ds, cudaStream_t s)
 {
-    k_auxi_dropin<double><<<node_grid(g), dim3(BX, BY), 0, s>>>(o, lsf, ahp, fin, g, ds);
+    k_auxi_dropin<<<node_grid(g), dim3(BX, BY), 0, s>>>(o, lsf, ahp, fin, g, tool64(g, ds));
     return cudaGetLastError();
 }
 

@@ -642,14 +642,6 @@ int op_aux_toolbox(const T *A, const T *F, T *const *out, int rows, int cols, in
     AuxKeep<T> keep = carve_aux<T>(b, g);
     AuxOut<T> o;
     for (int q = 0; q < AUX_OUT_FIELDS; ++q) o.f[q] = out[q];
-    // pass 2 reads the caller's arrays where the caller asked for those fields
-    if (o.f[4]) keep.cx = o.f[4];
-    if (o.f[5]) keep.cy = o.f[5];
-    if (o.f[6]) keep.cz = o.f[6];
-    if (o.f[7]) keep.ncr = o.f[7];
-    if (o.f[3]) keep.agm = o.f[3];
-    if (o.f[26]) keep.adelta = o.f[26];
-    if (o.f[25]) keep.aheav = o.f[25];
     VSL_TRY(launch_aux_toolbox<T>(A, F, o, keep, g, (dx + dy + dz) / 3, s));
     return VSL_OK;
 }

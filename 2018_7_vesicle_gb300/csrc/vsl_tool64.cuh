@@ -13,11 +13,12 @@
 namespace vsl {
 namespace {
 
-// the divisors of a grid
-struct Tool64 {
-    Divisor64 two[3], sq[3], four;  // 2 d, d d, (4 Ds) Ds
-    bool ordinary;
+// the divisors of a grid: 2 d, d d, (4 Ds) Ds
+template <typename D> struct ToolDivisors {
+    D two[3], sq[3], four;
+    bool ordinary;  // the spacings are within the range of the short quotients
 };
+using Tool64 = ToolDivisors<Divisor64>;
 inline Tool64 tool64(const Grid &g, double ds)
 {
     return Tool64{{divisor64(2 * g.dx), divisor64(2 * g.dy), divisor64(2 * g.dz)},
