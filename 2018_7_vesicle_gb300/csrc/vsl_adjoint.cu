@@ -24,9 +24,11 @@
 // differentiated.  The mask (sign of the field when a reinitialization starts) and the
 // fixed-node test are piecewise constant and carry no derivative.
 #include <cmath>
+#include <type_traits>
 
 #include "vsl_dual.cuh"
 #include "vsl_internal.h"
+#include "vsl_short64.cuh"
 
 namespace vsl {
 namespace {
@@ -55,16 +57,69 @@ __device__ __forceinline__ void adj_node_of(const Grid &g, long long c, int &i, 
     i = (int)(r - (long long)j * g.rows);
 }
 
+// Number types of the uniform stencils: quotients as a shared reciprocal, a product and a
+// remainder correction (vsl_short64.cuh), three to six instructions where a general quotient is
+// about twenty; a node took 38 of them per axis.  FP32: the hardware reciprocal is within an ulp,
+// and a Newton step from there gives the correctly rounded one, the quotient then too (Markstein's
+// theorems), so the values are those of general quotients.  Both need operands away from overflow
+// and underflow (uniform_range); other nodes take the general quotients.
+struct Short32 {
+    float v;
+    __device__ __forceinline__ Short32() {}
+    __device__ __forceinline__ Short32(float x) : v(x) {}
+    __device__ __forceinline__ Short32(double x) : v((float)x) {}
+    __device__ __forceinline__ Short32(int x) : v((float)x) {}
+    friend __device__ __forceinline__ Short32 operator+(Short32 a, Short32 b) { return a.v + b.v; }
+    friend __device__ __forceinline__ Short32 operator-(Short32 a, Short32 b) { return a.v - b.v; }
+    friend __device__ __forceinline__ Short32 operator*(Short32 a, Short32 b) { return a.v * b.v; }
+    friend __device__ __forceinline__ Short32 operator/(Short32 a, Short32 b)
+    {
+        const float y0 = rcp_ftz(b.v);
+        const float y = __fmaf_rn(__fmaf_rn(-b.v, y0, 1.f), y0, y0);
+        const float q = __fmul_rn(a.v, y);
+        return __fmaf_rn(__fmaf_rn(-b.v, q, a.v), y, q);
+    }
+};
+__device__ __forceinline__ float adj_raw(Short32 x) { return x.v; }
+__device__ __forceinline__ double adj_raw(Short64 x) { return x.v; }
+__device__ __forceinline__ float adj_raw(float x) { return x; }
+__device__ __forceinline__ double adj_raw(double x) { return x; }
+template <typename T> using ShortOf = typename std::conditional<std::is_same<T, float>::value, Short32, Short64>::type;
+
+// do the scaled differences of a line allow the short quotients
+__device__ __forceinline__ bool uniform_range(const float v[6])
+{
+    float m = 0.f;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) m = fmaxf(m, fabsf(v[q]));
+    bool nan = false;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) nan = nan || v[q] != v[q];
+    return m < 16384.f && !nan;
+}
+__device__ __forceinline__ bool uniform_range(const double v[6])
+{
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) ok = ok && within64(v[q], -200, 100);
+    return ok;
+}
+
 // Jiang-Shu WENO5 of five differences (the weno5_plain formula) and its gradient g[5]:
 // with alpha_k = d_k / (s_k + eps)^2 and w_k = alpha_k / sum alpha,
 //   dD/dv = sum_k w_k dq_k/dv + sum_k c_k ds_k/dv,   c_k = -2 w_k (q_k - D) / (s_k + eps),
 // where the candidates q_k are linear and the smoothness indicators s_k quadratic in v.
-template <typename T>
-__device__ __forceinline__ T weno5_grad(T v1, T v2, T v3, T v4, T v5, T g[5])
+// The candidates come in q (weno5_candidates).
+template <typename T> __device__ __forceinline__ void weno5_candidates(T v1, T v2, T v3, T v4, T v5, T q[3])
 {
-    const T q1 = T(1. / 3.) * v1 - T(7. / 6.) * v2 + T(11. / 6.) * v3;
-    const T q2 = T(-1. / 6.) * v2 + T(5. / 6.) * v3 + T(1. / 3.) * v4;
-    const T q3 = T(1. / 3.) * v3 + T(5. / 6.) * v4 - T(1. / 6.) * v5;
+    q[0] = T(1. / 3.) * v1 - T(7. / 6.) * v2 + T(11. / 6.) * v3;
+    q[1] = T(-1. / 6.) * v2 + T(5. / 6.) * v3 + T(1. / 3.) * v4;
+    q[2] = T(1. / 3.) * v3 + T(5. / 6.) * v4 - T(1. / 6.) * v5;
+}
+template <typename T>
+__device__ __forceinline__ T weno5_grad(T v1, T v2, T v3, T v4, T v5, const T q[3], T g[5])
+{
+    const T q1 = q[0], q2 = q[1], q3 = q[2];
     const T a1 = v1 - 2 * v2 + v3, b1 = v1 - 4 * v2 + 3 * v3;
     const T a2 = v2 - 2 * v3 + v4, b2 = v2 - v4;
     const T a3 = v3 - 2 * v4 + v5, b3 = 3 * v3 - 4 * v4 + v5;
@@ -91,27 +146,69 @@ __device__ __forceinline__ T weno5_grad(T v1, T v2, T v3, T v4, T v5, T g[5])
     return D;
 }
 
-// Uniform WENO5 pair of one axis line (weno5_pair_plain) with its partials with respect
-// to the seven line values: jf[o] = d D+ / d p[o], jb[o] = d D- / d p[o].
+// One side (back: D-, else D+) of the uniform WENO5 derivatives of an axis line with its partials
+// with respect to the seven line values: jac[o] = d D / d p[o].  A stage's update depends on one
+// side of an axis (the upwind one of a transport, the one that the Godunov norm took), so the other
+// side's partials, which would be multiplied by zero, are not formed.
+template <typename R, typename T>
+__device__ __forceinline__ void weno5_side_grad_of(const T v[6], bool back, T ih, T &D, T jac[7])
+{
+    // the candidates of both sides: with one side's alone the compiler would fuse other products
+    R g[5], qb[3], qf[3], q[3];
+    weno5_candidates<R>(R(v[0]), R(v[1]), R(v[2]), R(v[3]), R(v[4]), qb);
+    weno5_candidates<R>(R(v[5]), R(v[4]), R(v[3]), R(v[2]), R(v[1]), qf);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) q[m] = R(back ? adj_raw(qb[m]) : adj_raw(qf[m]));
+    D = adj_raw(weno5_grad<R>(R(back ? v[0] : v[5]), R(back ? v[1] : v[4]), R(back ? v[2] : v[3]),
+                              R(back ? v[3] : v[2]), R(back ? v[4] : v[1]), q, g));
+    // d D / d v[m], m = 0..5: g in the window's order
+    T G[6];
+    G[0] = back ? adj_raw(g[0]) : T(0);
+#pragma unroll
+    for (int m = 1; m < 5; ++m) G[m] = back ? adj_raw(g[m]) : adj_raw(g[5 - m]);
+    G[5] = back ? T(0) : adj_raw(g[0]);
+#pragma unroll
+    for (int o = 0; o < 7; ++o) {
+        const T l = o >= 1 ? G[o - 1] : T(0), r = o <= 5 ? G[o] : T(0);
+        jac[o] = (l - r) * ih;
+    }
+}
 template <typename T>
-__device__ __forceinline__ void weno5_pair_grad(const T p[7], T h, T &df, T &db, T jf[7], T jb[7])
+__device__ __noinline__ void weno5_side_grad_general(const T p[7], T h, bool back, T &D, T jac[7])
 {
     T v[6];
 #pragma unroll
     for (int m = 0; m < 6; ++m) v[m] = (p[m + 1] - p[m]) / h;
-    T gb[5], gf[5];
-    db = weno5_grad(v[0], v[1], v[2], v[3], v[4], gb);
-    df = weno5_grad(v[5], v[4], v[3], v[2], v[1], gf);
-    // G*[m] = d D / d v[m], m = 0..5
-    const T Gb[6] = {gb[0], gb[1], gb[2], gb[3], gb[4], T(0)};
-    const T Gf[6] = {T(0), gf[4], gf[3], gf[2], gf[1], gf[0]};
-    const T ih = T(1) / h;
+    weno5_side_grad_of<T>(v, back, T(1) / h, D, jac);
+}
+template <typename T> __device__ __forceinline__ void weno5_side_grad(const T p[7], T h, bool back, T &D, T jac[7])
+{
+    using R = ShortOf<T>;
+    T v[6];
 #pragma unroll
-    for (int o = 0; o < 7; ++o) {
-        const T lb = o >= 1 ? Gb[o - 1] : T(0), rb = o <= 5 ? Gb[o] : T(0);
-        const T lf = o >= 1 ? Gf[o - 1] : T(0), rf = o <= 5 ? Gf[o] : T(0);
-        jb[o] = (lb - rb) * ih;
-        jf[o] = (lf - rf) * ih;
+    for (int m = 0; m < 6; ++m) v[m] = adj_raw(R(p[m + 1] - p[m]) / R(h));
+    if (uniform_range(v))
+        weno5_side_grad_of<R>(v, back, adj_raw(R(T(1)) / R(h)), D, jac);
+    else
+        weno5_side_grad_general(p, h, back, D, jac);
+}
+
+// the uniform pair's values (weno5_pair_plain)
+template <typename T> __device__ __noinline__ void weno5_pair_general(const T p[7], T h, T &df, T &db)
+{
+    weno5_pair_plain<T>(p, h, df, db);
+}
+template <typename T> __device__ __forceinline__ void weno5_pair_values(const T p[7], T h, T &df, T &db)
+{
+    using R = ShortOf<T>;
+    T v[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) v[m] = adj_raw(R(p[m + 1] - p[m]) / R(h));
+    if (uniform_range(v)) {
+        db = adj_raw(weno5_plain<R>(v[0], v[1], v[2], v[3], v[4]));
+        df = adj_raw(weno5_plain<R>(v[5], v[4], v[3], v[2], v[1]));
+    } else {
+        weno5_pair_general(p, h, df, db);
     }
 }
 
@@ -151,15 +248,14 @@ __global__ void __launch_bounds__(BX *BY) k_adj_advect_jac(const T *__restrict__
     const T lc = coef * __ldg(lam + c) * (T)__ldg(dt);
 #pragma unroll 1
     for (int ax = 0; ax < 3; ++ax) {
-        T p[7], jf[7], jb[7], df, db;
+        T p[7], jac[7], D;
         load_line7(ps, axis_line(g, i, j, k, ax), p);
-        weno5_pair_grad<T>(p, (T)axis_h(g, ax), df, db, jf, jb);
+        // min(0, v) D+ + max(0, v) D-: D- where v > 0, D+ otherwise
         const T va = __ldg(v.p[ax] + c);
-        const T vm = vmin(T(0), va), vp = vmax(T(0), va);
+        weno5_side_grad<T>(p, (T)axis_h(g, ax), va > T(0), D, jac);
 #pragma unroll
-        for (int o = 0; o < 7; ++o) W[(long long)(ax * 7 + o) * g.num + c] = lc * (vm * jf[o] + vp * jb[o]);
-        // d step / d v: D- where v > 0, D+ otherwise (the branches of max/min above)
-        gv.p[ax][c] -= lc * (va > T(0) ? db : df);
+        for (int o = 0; o < 7; ++o) W[(long long)(ax * 7 + o) * g.num + c] = lc * (va * jac[o]);
+        gv.p[ax][c] -= lc * D;
     }
 }
 
@@ -202,7 +298,7 @@ __device__ __forceinline__ void reinit_jac_node(const T *__restrict__ ps, const 
         if (GENERIC && iface[ax])
             interface_pair<T>(p, dist[2 * ax], dist[2 * ax + 1], h[ax], T(0), T(0), false, df, db);
         else
-            weno5_pair_plain<T>(p, h[ax], df, db);
+            weno5_pair_values<T>(p, h[ax], df, db);
         const T A = neg ? sqr(vmin(z, db)) : sqr(vmax(z, db));
         const T B = neg ? sqr(vmax(z, df)) : sqr(vmin(z, df));
         if (A < B) {  // vmax(A, B) took B (the forward derivative)
@@ -223,24 +319,26 @@ __device__ __forceinline__ void reinit_jac_node(const T *__restrict__ ps, const 
     T md[6];
 #pragma unroll 1
     for (int ax = 0; ax < 3; ++ax) {
-        T p[7], jf[9], jb[9], df, db;
+        T p[7];
         load_line7(ps, axis_line(g, i, j, k, ax), p);
-        if constexpr (GENERIC) {
-            if (iface[ax]) {
-                iface_pair_jac<T>(p, h[ax], dist[2 * ax], dist[2 * ax + 1], df, db, jf, jb);
-            } else {
-                weno5_pair_grad<T>(p, h[ax], df, db, jf, jb);
-                jf[7] = jf[8] = jb[7] = jb[8] = T(0);
-            }
-        } else {
-            weno5_pair_grad<T>(p, h[ax], df, db, jf, jb);
-            jf[7] = jf[8] = jb[7] = jb[8] = T(0);
-        }
         const T gf = gq[2 * ax] * dG * s_dt, gb = gq[2 * ax + 1] * dG * s_dt;
+        md[2 * ax] = md[2 * ax + 1] = T(0);
+        if (GENERIC && iface[ax]) {
+            T jf[9], jb[9], df, db;
+            iface_pair_jac<T>(p, h[ax], dist[2 * ax], dist[2 * ax + 1], df, db, jf, jb);
 #pragma unroll
-        for (int o = 0; o < 7; ++o) W[(long long)(ax * 7 + o) * g.num + c] = lc * (gf * jf[o] + gb * jb[o]);
-        md[2 * ax] = gf * jf[7] + gb * jb[7];
-        md[2 * ax + 1] = gf * jf[8] + gb * jb[8];
+            for (int o = 0; o < 7; ++o) W[(long long)(ax * 7 + o) * g.num + c] = lc * (gf * jf[o] + gb * jb[o]);
+            md[2 * ax] = gf * jf[7] + gb * jb[7];
+            md[2 * ax + 1] = gf * jf[8] + gb * jb[8];
+        } else {
+            // the norm took one side: gf or gb is zero
+            T jac[7], D;
+            const bool back = gf == T(0);
+            weno5_side_grad<T>(p, h[ax], back, D, jac);
+            const T gs = back ? gb : gf;
+#pragma unroll
+            for (int o = 0; o < 7; ++o) W[(long long)(ax * 7 + o) * g.num + c] = lc * (gs * jac[o]);
+        }
     }
     // d step / d dist_q: through the interface insertion, and through dt for the minimum
 #pragma unroll

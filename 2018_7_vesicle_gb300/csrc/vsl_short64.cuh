@@ -47,6 +47,7 @@ struct Short64 {
     double v;
     __device__ __forceinline__ Short64() {}
     __device__ __forceinline__ Short64(double x) : v(x) {}
+    __device__ __forceinline__ Short64(int x) : v((double)x) {}
     friend __device__ __forceinline__ Short64 operator+(Short64 a, Short64 b) { return __dadd_rn(a.v, b.v); }
     friend __device__ __forceinline__ Short64 operator-(Short64 a, Short64 b) { return __dadd_rn(a.v, -b.v); }
     friend __device__ __forceinline__ Short64 operator-(Short64 a) { return -a.v; }
