@@ -57,6 +57,27 @@ __device__ __forceinline__ void adj_node_of(const Grid &g, long long c, int &i, 
     i = (int)(r - (long long)j * g.rows);
 }
 
+// products rounded by themselves, as where the forward code kept them in arrays
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// the seven values of an axis line through node c; lines away from the faces take no clamps
+template <typename T>
+__device__ __forceinline__ void adj_line7(const T *__restrict__ f, const Grid &g, int i, int j, int k, long long c,
+                                          int ax, T p[7])
+{
+    const int q = ax == AX_X ? j : (ax == AX_Y ? i : k), n = ax == AX_X ? g.cols : (ax == AX_Y ? g.rows : g.pges);
+    const long long stride = ax == AX_X ? (long long)g.rows : (ax == AX_Y ? 1 : g.plane);
+    const T *fc = f + c;
+    if (q >= 3 && q + 3 < n) {
+#pragma unroll
+        for (int s = -3; s <= 3; ++s) p[s + 3] = __ldg(fc + s * stride);
+    } else {
+#pragma unroll
+        for (int s = -3; s <= 3; ++s) p[s + 3] = __ldg(fc + (clampi(q + s, n) - q) * stride);
+    }
+}
+
 // Number types of the uniform stencils: quotients as a shared reciprocal, a product and a
 // remainder correction (vsl_short64.cuh), three to six instructions where a general quotient is
 // about twenty; a node took 38 of them per axis.  FP32: the hardware reciprocal is within an ulp,
@@ -86,16 +107,17 @@ __device__ __forceinline__ float adj_raw(float x) { return x; }
 __device__ __forceinline__ double adj_raw(double x) { return x; }
 template <typename T> using ShortOf = typename std::conditional<std::is_same<T, float>::value, Short32, Short64>::type;
 
-// do the scaled differences of a line allow the short quotients
+// do the scaled differences of a line allow the short quotients (NaN fails the comparison)
+__device__ __forceinline__ float max3_nan(float a, float b, float c)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 __device__ __forceinline__ bool uniform_range(const float v[6])
 {
-    float m = 0.f;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) m = fmaxf(m, fabsf(v[q]));
-    bool nan = false;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) nan = nan || v[q] != v[q];
-    return m < 16384.f && !nan;
+    const float m = max3_nan(fabsf(v[0]), fabsf(v[1]), fabsf(v[2])), n = max3_nan(fabsf(v[3]), fabsf(v[4]), fabsf(v[5]));
+    return max3_nan(m, n, n) < 16384.f;
 }
 __device__ __forceinline__ bool uniform_range(const double v[6])
 {
@@ -212,32 +234,40 @@ template <typename T> __device__ __forceinline__ void weno5_pair_values(const T 
     }
 }
 
-// Interface-aware pair (nonuniform WENO5 with the interface inserted at r1 / l1, value 0)
-// and its partials with respect to the seven line values (0..6) and r1, l1 (7, 8), by
-// dual numbers; out of line, since only the few band nodes take it.
+// One side (back: D-, else D+) of the nonuniform WENO5 pair, out of line on dual numbers.
+template <typename D> __device__ __noinline__ D nonuniform_side(const D xs[7], const D hs[7], bool back)
+{
+    D dd[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) dd[m] = (hs[m + 1] - hs[m]) / (xs[m + 1] - xs[m]);
+    if (back) return weno_nonuniform_back<D>(xs, dd);
+    return weno_nonuniform_fore<D>(xs, dd);
+}
+
+// One side of the interface-aware pair (nonuniform WENO5 with the interface inserted at r1 / l1,
+// value 0): its partials with respect to the seven line values (0..6) and r1, l1 (7, 8), by dual
+// numbers.
 template <typename T>
-__device__ __noinline__ void iface_pair_jac(const T p[7], T h, T r1, T l1, T &df, T &db, T jf[9], T jb[9])
+__device__ __noinline__ void iface_side_jac(const T p[7], T h, T r1, T l1, bool back, T jac[9])
 {
     using D = Dual<T, 9>;
-    D P[7];
+    D P[7], xs[7], hs[7];
 #pragma unroll
     for (int o = 0; o < 7; ++o) P[o] = D::var(p[o], o);
-    D f, b;
-    interface_pair<D>(P, D::var(r1, 7), D::var(l1, 8), D((double)h), D(0.0), D(0.0), false, f, b);
-    df = f.v;
-    db = b.v;
+    insert_interface<D>(P, D::var(r1, 7), D::var(l1, 8), D((double)h), D(0.0), D(0.0), xs, hs);
+    const D r = nonuniform_side<D>(xs, hs, back);
 #pragma unroll
-    for (int o = 0; o < 9; ++o) {
-        jf[o] = f.d[o];
-        jb[o] = b.d[o];
-    }
+    for (int o = 0; o < 9; ++o) jac[o] = r.d[o];
 }
 
 // ---------------------------------------------------------------------------------------
 // advection stage: step = dt * sum_ax (min(0, v) D+ + max(0, v) D-)  (uniform WENO5)
+// Bound by its instructions (about 1000 per node, 60 % of the issue slots) and the 176 MB of slots
+// that it writes at 128^3 (30 % of the memory rate).  The next axis' line and velocity adjoint are
+// loaded while an axis is formed, and the slots' addresses advance by additions: 105 -> 93 us.
 // ---------------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(BX *BY) k_adj_advect_jac(const T *__restrict__ ps, Ptr3<const T> v,
+__global__ void __launch_bounds__(BX *BY, 5) k_adj_advect_jac(const T *__restrict__ ps, Ptr3<const T> v,
                                                              const double *__restrict__ dt,
                                                              const T *__restrict__ lam, T coef, T *__restrict__ W,
                                                              Ptr3<T> gv, Grid g)
@@ -246,107 +276,104 @@ __global__ void __launch_bounds__(BX *BY) k_adj_advect_jac(const T *__restrict__
     long long c;
     if (!adj_node(g, i, j, k, c)) return;
     const T lc = coef * __ldg(lam + c) * (T)__ldg(dt);
+    T p[7], va = __ldg(v.p[0] + c), ga = gv.p[0][c];
+    T *w = W + c;
+    adj_line7(ps, g, i, j, k, c, 0, p);
 #pragma unroll 1
     for (int ax = 0; ax < 3; ++ax) {
-        T p[7], jac[7], D;
-        load_line7(ps, axis_line(g, i, j, k, ax), p);
+        // the next axis is on its way while this one is formed
+        T pn[7], vn, gn;
+        if (ax < 2) {
+            adj_line7(ps, g, i, j, k, c, ax + 1, pn);
+            vn = __ldg(v.p[ax + 1] + c);
+            gn = gv.p[ax + 1][c];
+        }
         // min(0, v) D+ + max(0, v) D-: D- where v > 0, D+ otherwise
-        const T va = __ldg(v.p[ax] + c);
+        T jac[7], D;
         weno5_side_grad<T>(p, (T)axis_h(g, ax), va > T(0), D, jac);
 #pragma unroll
-        for (int o = 0; o < 7; ++o) W[(long long)(ax * 7 + o) * g.num + c] = lc * (va * jac[o]);
-        gv.p[ax][c] -= lc * D;
+        for (int o = 0; o < 7; ++o, w += g.num) *w = lc * (va * jac[o]);
+        gv.p[ax][c] = ga - lc * D;
+#pragma unroll
+        for (int o = 0; o < 7; ++o) p[o] = pn[o];
+        va = vn;
+        ga = gn;
     }
 }
 
 // ---------------------------------------------------------------------------------------
 // reinitialization stage: step = (|grad|_Godunov - 1) * 0.3 min(dist) * (mask ? -1 : 1)
 // ---------------------------------------------------------------------------------------
-// One node of the reinitialization-stage Jacobian.  GENERIC = false handles only nodes
-// whose three axis lines are all uniform (no sign change next to the node); GENERIC =
-// true also differentiates the interface-aware pairs (dual numbers) and is run over the
-// compact list of the remaining nodes, so the register cost of the dual code does not
-// limit the occupancy of the dense pass.
-template <typename T, bool GENERIC>
+// the six distances (stored where flagged, the spacing elsewhere) and their minimum (the
+// pseudo-time step is 0.3 times it), taken in the order of the forward kernel's vmin tree
+template <typename T>
+__device__ __forceinline__ int reinit_distances(uint8_t fl, const Ptr6<const T> &d, long long c, const Grid &g, T dist[6])
+{
+    const T h[3] = {(T)g.dx, (T)g.dy, (T)g.dz};
+#pragma unroll
+    for (int q = 0; q < 6; ++q) dist[q] = (fl & (1u << q)) ? __ldg(d.p[q] + c) : h[q / 2];
+    const T d01 = dist[0] < dist[1] ? dist[0] : dist[1], d23 = dist[2] < dist[3] ? dist[2] : dist[3],
+            d45 = dist[4] < dist[5] ? dist[4] : dist[5], d25 = d23 < d45 ? d23 : d45;
+    const int i01 = dist[0] < dist[1] ? 0 : 1, i23 = dist[2] < dist[3] ? 2 : 3, i45 = dist[4] < dist[5] ? 4 : 5;
+    return d01 < d25 ? i01 : (d23 < d45 ? i23 : i45);
+}
+
+// One axis of the Godunov norm G = sqrt(sum_ax max(A_ax, B_ax)), with the branch of the max as
+// the forward took it: the squared term, the side taken (back: D-) and the derivative gs of the
+// term with respect to that side.
+template <typename T> __device__ __forceinline__ T godunov_axis(bool neg, T df, T db, T &gs, bool &back)
+{
+    const T z = T(0);
+    const T A = neg ? sqr(vmin(z, db)) : sqr(vmax(z, db));
+    const T B = neg ? sqr(vmax(z, df)) : sqr(vmin(z, df));
+    back = !(A < B);
+    gs = T(2) * (back ? (neg ? vmin(z, db) : vmax(z, db)) : (neg ? vmax(z, df) : vmin(z, df)));
+    return back ? A : B;
+}
+
+// One node of the reinitialization-stage Jacobian whose three axis lines are all uniform (no sign
+// change next to the node).
+template <typename T>
 __device__ __forceinline__ void reinit_jac_node(const T *__restrict__ ps, const uint8_t fl, Ptr6<const T> d,
                                                 const T lc, T *__restrict__ W, Ptr6<T> mu, const Grid &g, int i,
                                                 int j, int k, long long c)
 {
-    const T h[3] = {(T)g.dx, (T)g.dy, (T)g.dz};
-    // the six distances (stored where flagged, the spacing elsewhere); the pseudo-time
-    // step is 0.3 * their minimum, taken in the order of the forward kernel's vmin tree
     T dist[6];
+    const int qmin = reinit_distances(fl, d, c, g, dist);
+    T dmin = dist[0];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) dist[q] = (fl & (1u << q)) ? __ldg(d.p[q] + c) : h[q / 2];
-    const int i01 = dist[0] < dist[1] ? 0 : 1, i23 = dist[2] < dist[3] ? 2 : 3, i45 = dist[4] < dist[5] ? 4 : 5;
-    const int i25 = dist[i23] < dist[i45] ? i23 : i45;
-    const int qmin = dist[i01] < dist[i25] ? i01 : i25;
-    const T dtv = T(0.3) * dist[qmin];
+    for (int q = 1; q < 6; ++q) dmin = q == qmin ? dist[q] : dmin;
+    const T dtv = T(0.3) * dmin;
     const bool neg = fl & CLS_MASK;
     const T sgn = neg ? T(-1) : T(1);
 
     // pass 1: the derivative pairs and the partials of the Godunov norm
-    //   G = sqrt(sum_ax max(A_ax, B_ax)) with the branch of each max as the forward took it
-    bool iface[3];
-    T gq[6], S = T(0);
-    const T z = T(0);
+    T gq[3], S = T(0);
+    bool back[3];
 #pragma unroll 1
     for (int ax = 0; ax < 3; ++ax) {
         T p[7], df, db;
-        load_line7(ps, axis_line(g, i, j, k, ax), p);
-        iface[ax] = GENERIC && (p[2] * p[3] < T(0) || p[3] * p[4] < T(0));
-        if (GENERIC && iface[ax])
-            interface_pair<T>(p, dist[2 * ax], dist[2 * ax + 1], h[ax], T(0), T(0), false, df, db);
-        else
-            weno5_pair_values<T>(p, h[ax], df, db);
-        const T A = neg ? sqr(vmin(z, db)) : sqr(vmax(z, db));
-        const T B = neg ? sqr(vmax(z, df)) : sqr(vmin(z, df));
-        if (A < B) {  // vmax(A, B) took B (the forward derivative)
-            S += B;
-            gq[2 * ax] = T(2) * (neg ? vmax(z, df) : vmin(z, df));
-            gq[2 * ax + 1] = T(0);
-        } else {
-            S += A;
-            gq[2 * ax] = T(0);
-            gq[2 * ax + 1] = T(2) * (neg ? vmin(z, db) : vmax(z, db));
-        }
+        adj_line7(ps, g, i, j, k, c, ax, p);
+        weno5_pair_values<T>(p, (T)axis_h(g, ax), df, db);
+        S = add_rn(S, godunov_axis(neg, df, db, gq[ax], back[ax]));
     }
     const T G = sqrt(S);
     const T dG = G > T(0) ? T(0.5) / G : T(0);  // zero derivative of sqrt at 0
     const T s_dt = dtv * sgn;
 
-    // pass 2: per axis, partials of the pair, scaled into the slots and distance adjoints
-    T md[6];
+    // pass 2: per axis, partials of the side taken, scaled into the slots
+    T *w = W + c;
 #pragma unroll 1
     for (int ax = 0; ax < 3; ++ax) {
-        T p[7];
-        load_line7(ps, axis_line(g, i, j, k, ax), p);
-        const T gf = gq[2 * ax] * dG * s_dt, gb = gq[2 * ax + 1] * dG * s_dt;
-        md[2 * ax] = md[2 * ax + 1] = T(0);
-        if (GENERIC && iface[ax]) {
-            T jf[9], jb[9], df, db;
-            iface_pair_jac<T>(p, h[ax], dist[2 * ax], dist[2 * ax + 1], df, db, jf, jb);
+        T p[7], jac[7], D;
+        adj_line7(ps, g, i, j, k, c, ax, p);
+        const T gs = gq[ax] * dG * s_dt;
+        weno5_side_grad<T>(p, (T)axis_h(g, ax), back[ax], D, jac);
 #pragma unroll
-            for (int o = 0; o < 7; ++o) W[(long long)(ax * 7 + o) * g.num + c] = lc * (gf * jf[o] + gb * jb[o]);
-            md[2 * ax] = gf * jf[7] + gb * jb[7];
-            md[2 * ax + 1] = gf * jf[8] + gb * jb[8];
-        } else {
-            // the norm took one side: gf or gb is zero
-            T jac[7], D;
-            const bool back = gf == T(0);
-            weno5_side_grad<T>(p, h[ax], back, D, jac);
-            const T gs = back ? gb : gf;
-#pragma unroll
-            for (int o = 0; o < 7; ++o) W[(long long)(ax * 7 + o) * g.num + c] = lc * (gs * jac[o]);
-        }
+        for (int o = 0; o < 7; ++o, w += g.num) *w = lc * (gs * jac[o]);
     }
-    // d step / d dist_q: through the interface insertion, and through dt for the minimum
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        if (!(fl & (1u << q))) continue;
-        const T ds = md[q] + (q == qmin ? (G - T(1)) * sgn * T(0.3) : T(0));
-        mu.p[q][c] -= lc * ds;
-    }
+    // d step / d dist_q: through dt for the minimum
+    if (fl & (1u << qmin)) mu.p[qmin][c] -= lc * ((G - T(1)) * sgn * T(0.3));
 }
 
 // warp-aggregated append of `value` where `pred` holds (all 32 lanes of the warp call it)
@@ -391,61 +418,172 @@ __global__ void __launch_bounds__(BX *BY) k_adj_reinit_jac(const T *__restrict__
         for (int s = 0; s < SLOTS; ++s) W[(long long)s * g.num + c] = T(0);
         return;
     }
-    reinit_jac_node<T, false>(ps, fl, d, coef * __ldg(lam + c), W, mu, g, i, j, k, c);
+    reinit_jac_node<T>(ps, fl, d, coef * __ldg(lam + c), W, mu, g, i, j, k, c);
 }
 
+// The listed nodes (40,000 around a sphere of radius 38), BAND_NODES at a time, as (node, axis) tasks: the derivative pairs first, then,
+// once the norm of each node is known, the partials, with the tasks in order of kind (uniform,
+// interface-aware forward, interface-aware backward) so that a warp takes one path.  Bound by
+// fetching the instructions of the dual-number code, eight warps to a multiprocessor (255
+// registers).  A thread per node with both sides of three axes took 110 us, a task to a lane
+// without the order 89, this 76 (42 nodes to a block of 128: 77).
+constexpr int BAND_NODES = 85, BAND_THREADS = 256;
 template <typename T>
-__global__ void __launch_bounds__(128) k_adj_reinit_jac_band(const T *__restrict__ ps,
-                                                               const uint8_t *__restrict__ flags, Ptr6<const T> d,
-                                                               const T *__restrict__ lam, T coef, T *__restrict__ W,
-                                                               Ptr6<T> mu, NodeList band, Grid g)
+__global__ void __launch_bounds__(BAND_THREADS) k_adj_reinit_jac_band(const T *__restrict__ ps,
+                                                                        const uint8_t *__restrict__ flags,
+                                                                        Ptr6<const T> d, const T *__restrict__ lam,
+                                                                        T coef, T *__restrict__ W, Ptr6<T> mu,
+                                                                        NodeList band, Grid g)
 {
+    __shared__ T sdf[BAND_NODES][3], sdb[BAND_NODES][3];
+    __shared__ unsigned char order[3 * BAND_NODES];
+    __shared__ int kinds[4];
+    const int tid = threadIdx.x;
     const unsigned n = *band.count;
-    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const long long c = band.idx[t];
-        int i, j, k;
-        adj_node_of(g, c, i, j, k);
-        reinit_jac_node<T, true>(ps, __ldg(flags + c), d, coef * __ldg(lam + c), W, mu, g, i, j, k, c);
+    for (unsigned t0 = blockIdx.x * BAND_NODES; t0 < n; t0 += gridDim.x * BAND_NODES) {
+        const int nodes = min((unsigned)BAND_NODES, n - t0);
+        const bool task = tid < 3 * nodes;
+        if (tid < 4) kinds[tid] = 0;
+        __syncthreads();
+        int kind = 0, rank = 0;
+        if (task) {
+            const int q = tid / 3, ax = tid - 3 * q;
+            const long long c = band.idx[t0 + q];
+            int i, j, k;
+            adj_node_of(g, c, i, j, k);
+            const uint8_t fl = __ldg(flags + c);
+            const T h = (T)axis_h(g, ax);
+            T p[7], df, db, gs;
+            bool back;
+            adj_line7(ps, g, i, j, k, c, ax, p);
+            const bool iface = p[2] * p[3] < T(0) || p[3] * p[4] < T(0);
+            if (iface) {
+                const T r1 = (fl & (1u << (2 * ax))) ? __ldg(d.p[2 * ax] + c) : h;
+                const T l1 = (fl & (2u << (2 * ax))) ? __ldg(d.p[2 * ax + 1] + c) : h;
+                interface_pair<T>(p, r1, l1, h, T(0), T(0), false, df, db);
+            } else {
+                weno5_pair_values<T>(p, h, df, db);
+            }
+            godunov_axis((fl & CLS_MASK) != 0, df, db, gs, back);
+            sdf[q][ax] = df;
+            sdb[q][ax] = db;
+            kind = iface ? (back ? 2 : 1) : 0;
+            rank = atomicAdd(kinds + kind, 1);
+        }
+        __syncthreads();
+        if (task) order[rank + (kind > 0 ? kinds[0] : 0) + (kind > 1 ? kinds[1] : 0)] = (unsigned char)tid;
+        __syncthreads();
+        if (task) {
+            const int q = order[tid] / 3, ax = order[tid] - 3 * q;
+            const bool iface = tid >= kinds[0], back_side = tid >= kinds[0] + kinds[1];
+            const long long c = band.idx[t0 + q];
+            int i, j, k;
+            adj_node_of(g, c, i, j, k);
+            const uint8_t fl = __ldg(flags + c);
+            const bool neg = fl & CLS_MASK;
+            const T sgn = neg ? T(-1) : T(1), h = (T)axis_h(g, ax), lc = coef * __ldg(lam + c);
+            T dist[6], p[7];
+            const int qmin = reinit_distances(fl, d, c, g, dist);
+            adj_line7(ps, g, i, j, k, c, ax, p);
+            T dmin = dist[0], r1 = dist[0], l1 = dist[1];
+#pragma unroll
+            for (int m = 1; m < 6; ++m) dmin = m == qmin ? dist[m] : dmin;
+#pragma unroll
+            for (int a = 1; a < 3; ++a) {
+                r1 = a == ax ? dist[2 * a] : r1;
+                l1 = a == ax ? dist[2 * a + 1] : l1;
+            }
+            T S = T(0), gs = T(0);
+            bool back = false;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                T ga;
+                bool ba;
+                S = add_rn(S, godunov_axis(neg, sdf[q][a], sdb[q][a], ga, ba));
+                gs = a == ax ? ga : gs;
+                back = a == ax ? ba : back;
+            }
+            const T G = sqrt(S);
+            const T dG = G > T(0) ? T(0.5) / G : T(0);  // zero derivative of sqrt at 0
+            gs = gs * dG * (T(0.3) * dmin * sgn);
+            T jac[9];
+            if (iface) {
+                iface_side_jac<T>(p, h, r1, l1, back_side, jac);
+            } else {
+                T D;
+                weno5_side_grad<T>(p, h, back, D, jac);
+                jac[7] = jac[8] = T(0);
+            }
+            T *w = W + (long long)(ax * 7) * g.num + c;
+#pragma unroll
+            for (int o = 0; o < 7; ++o, w += g.num) *w = lc * (gs * jac[o]);
+            // d step / d dist: through the interface insertion, and through dt for the minimum
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const int m = 2 * ax + o;
+                const T md = mul_rn(gs, jac[7 + o]);
+                const T ds = md + (m == qmin ? (G - T(1)) * sgn * T(0.3) : T(0));
+                if (fl & (1u << m)) mu.p[m][c] -= lc * ds;
+            }
+        }
+        __syncthreads();
     }
 }
 
 // ---------------------------------------------------------------------------------------
 // transpose pass: out_j = alpha * lam_j - sum of W over the stencil positions equal to j
 // (+ acc_j)
+// Bound by memory: 185 MB of slots at 128^3, 42 us (4.4 TB/s beside the write-back of the slots);
+// with clamped 64-bit index arithmetic and first pages first it took 54.
 // ---------------------------------------------------------------------------------------
+// offset of the source of slot ax*7+o from its node: its slot's array, o - 3 nodes back
+struct GatherOffsets {
+    long long at[SLOTS];
+};
 template <typename T>
 __global__ void __launch_bounds__(BX *BY) k_adj_gather(const T *__restrict__ W, const T *lam, T alpha,
-                                                         const T *__restrict__ acc, T *out, Grid g)
+                                                         const T *__restrict__ acc, T *out, GatherOffsets from, Grid g)
 {
-    int i, j, k;
-    long long c;
-    if (!adj_node(g, i, j, k, c)) return;
-    T s = T(0);
-#pragma unroll 1
+    // last pages first: theirs are the slots that the pass before wrote last, still in L2
+    const int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y, k = gridDim.z - 1 - blockIdx.z;
+    if (i >= g.rows || j >= g.cols) return;
+    const long long c = node_index(g, i, j, k);
+    // sources whose offset o lands exactly on the node (none beyond an edge), all on their way at once
+    T w[3][7];
+    const T *Wc = W + c;
+#pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
-        const AxisLine L = axis_line(g, i, j, k, ax);
-        const T *Wa = W + (long long)(ax * 7) * g.num + L.base;
-        const int cj = L.c, n = L.n;
-        s += Wa[3 * g.num + (long long)cj * L.stride];
-        // sources whose offset o lands exactly on cj
+        const int cj = ax == AX_X ? j : (ax == AX_Y ? i : k), n = ax == AX_X ? g.cols : (ax == AX_Y ? g.rows : g.pges);
 #pragma unroll
         for (int o = 0; o < 7; ++o) {
-            if (o == 3) continue;
-            const int ci = cj - (o - 3);
-            if (ci >= 0 && ci < n) s += Wa[(long long)o * g.num + (long long)ci * L.stride];
-        }
-        // sources whose offset ran past an edge and was clamped onto cj
-        if (cj == 0) {
-            for (int ci = 0; ci < min(3, n); ++ci)
-                for (int o = 0; o <= 2 - ci; ++o) s += Wa[(long long)o * g.num + (long long)ci * L.stride];
-        }
-        if (cj == n - 1) {
-            for (int ci = max(0, n - 3); ci < n; ++ci)
-                for (int o = n + 3 - ci; o <= 6; ++o) s += Wa[(long long)o * g.num + (long long)ci * L.stride];
+            const bool in = o < 3 ? cj + (3 - o) < n : (o > 3 ? cj >= o - 3 : true);
+            w[ax][o] = in ? __ldg(Wc + from.at[ax * 7 + o]) : T(0);
         }
     }
-    const T a = acc ? acc[c] : T(0);
-    out[c] = alpha * lam[c] - s + a;
+    const T l = lam[c], a = acc ? acc[c] : T(0);
+    T s = T(0);
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        const int cj = ax == AX_X ? j : (ax == AX_Y ? i : k), n = ax == AX_X ? g.cols : (ax == AX_Y ? g.rows : g.pges);
+        const long long stride = ax == AX_X ? (long long)g.rows : (ax == AX_Y ? 1 : g.plane);
+        const T *Wa = W + (long long)(ax * 7) * g.num + c;
+        s += w[ax][3];
+#pragma unroll
+        for (int o = 0; o < 7; ++o)
+            if (o != 3) s += w[ax][o];
+        // sources whose offset ran past an edge and was clamped onto cj
+        if (cj == 0) {
+#pragma unroll 1
+            for (int ci = 0; ci < min(3, n); ++ci)
+                for (int o = 0; o <= 2 - ci; ++o) s += Wa[(long long)o * g.num + ci * stride];
+        }
+        if (cj == n - 1) {
+#pragma unroll 1
+            for (int ci = max(0, n - 3); ci < n; ++ci)
+                for (int o = n + 3 - ci; o <= 6; ++o) s += Wa[(long long)o * g.num + (ci - cj) * stride];
+        }
+    }
+    out[c] = alpha * l - s + a;
 }
 
 // acc = (init ? 0 : acc) + a * lam
@@ -563,7 +701,7 @@ cudaError_t launch_adj_reinit_jac(const T *ps, const uint8_t *flags, Ptr6<const 
     cudaError_t err = cudaMemsetAsync(band.count, 0, sizeof(unsigned), s);
     if (err != cudaSuccess) return err;
     k_adj_reinit_jac<T><<<node_grid(g), dim3(BX, BY), 0, s>>>(ps, flags, d, lam, (T)coef, W, mu, band, g);
-    k_adj_reinit_jac_band<T><<<adj_list_blocks(), 128, 0, s>>>(ps, flags, d, lam, (T)coef, W, mu, band, g);
+    k_adj_reinit_jac_band<T><<<adj_list_blocks(), BAND_THREADS, 0, s>>>(ps, flags, d, lam, (T)coef, W, mu, band, g);
     return cudaGetLastError();
 }
 
@@ -571,7 +709,10 @@ template <typename T>
 cudaError_t launch_adj_gather(const T *W, const T *lam, double alpha, const T *acc, T *out, const Grid &g,
                               cudaStream_t s)
 {
-    k_adj_gather<T><<<node_grid(g), dim3(BX, BY), 0, s>>>(W, lam, (T)alpha, acc, out, g);
+    const long long stride[3] = {g.rows, 1, g.plane};
+    GatherOffsets from;
+    for (int q = 0; q < SLOTS; ++q) from.at[q] = q * g.num - (q % 7 - 3) * stride[q / 7];
+    k_adj_gather<T><<<node_grid(g), dim3(BX, BY), 0, s>>>(W, lam, (T)alpha, acc, out, from, g);
     return cudaGetLastError();
 }
 

@@ -50,3 +50,41 @@ def test_quotients_round_correctly(tmp_path, kind):
     lib = ctypes.CDLL(str(so))
     lib.check.restype, lib.check.argtypes = ctypes.c_long, [ctypes.c_long, ctypes.c_int]
     assert lib.check(4_000_000, kind) == 0
+
+
+# The FP32 quotient of the adjoint's uniform stencils (csrc/vsl_adjoint.cu): a Newton step from a
+# reciprocal that is off by up to an ulp, and the same remainder correction.
+SRC32 = r"""
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+static uint32_t s = 2463534242u;
+static uint32_t rnd(void) { s ^= s << 13; s ^= s >> 17; s ^= s << 5; return s; }
+static float bits(uint32_t m, int e) { return ldexpf((float)((m & 0x7fffff) | 0x800000), e - 23); }
+long check(long n) {
+    long bad = 0;
+    for (long k = 0; k < n; ++k) {
+        float b = bits(k % 8 == 0 ? 0x7fffffu - rnd() % 4 : (k % 8 == 1 ? rnd() % 4 : rnd()), (int)(rnd() % 40) - 20);
+        float a = bits(rnd(), (int)(rnd() % 40) - 20);
+        if (k % 4 == 2) a = fmaf(bits(rnd(), 0), b, 0.5f * ldexpf(b, -23));
+        if (k % 16 == 3) a = 0.f;
+        if (k % 3 == 0) a = -a;
+        float y0 = 1.f / b;
+        y0 = k % 5 < 2 ? nextafterf(y0, 0.f) : (k % 5 < 4 ? nextafterf(y0, INFINITY) : y0);
+        float y = fmaf(fmaf(-b, y0, 1.f), y0, y0), q = a * y;
+        volatile float want = a / b;
+        if (fmaf(fmaf(-b, q, a), y, q) != want) ++bad;
+    }
+    return bad;
+}
+"""
+
+
+def test_fp32_quotients_round_correctly(tmp_path):
+    (tmp_path / "q32.c").write_text(SRC32)
+    so = tmp_path / "q32.so"
+    subprocess.run(["gcc", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-o", str(so), str(tmp_path / "q32.c"),
+                    "-lm"], check=True)
+    lib = ctypes.CDLL(str(so))
+    lib.check.restype, lib.check.argtypes = ctypes.c_long, [ctypes.c_long]
+    assert lib.check(8_000_000) == 0
