@@ -331,12 +331,38 @@ template <typename T> __device__ __forceinline__ T godunov_axis(bool neg, T df, 
     return back ? A : B;
 }
 
+// One axis of a uniform line p: the term of the Godunov norm with its derivative gs with respect
+// to the side that the norm takes, and that side's partials.
+template <typename T>
+__device__ __forceinline__ T reinit_axis(const T p[7], T h, bool neg, T &gs, T jac[7])
+{
+    using R = ShortOf<T>;
+    T v[6], D, df, db;
+    bool back;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) v[m] = adj_raw(R(p[m + 1] - p[m]) / R(h));
+    const bool in_range = uniform_range(v);
+    if (in_range) {
+        db = adj_raw(weno5_plain<R>(v[0], v[1], v[2], v[3], v[4]));
+        df = adj_raw(weno5_plain<R>(v[5], v[4], v[3], v[2], v[1]));
+    } else {
+        weno5_pair_general(p, h, df, db);
+    }
+    const T X = godunov_axis(neg, df, db, gs, back);
+    if (in_range)
+        weno5_side_grad_of<R>(v, back, adj_raw(R(T(1)) / R(h)), D, jac);
+    else
+        weno5_side_grad_general(p, h, back, D, jac);
+    return X;
+}
+
 // One node of the reinitialization-stage Jacobian whose three axis lines are all uniform (no sign
-// change next to the node).
+// change next to the node).  An axis is visited once: its side's partials wait in shared memory
+// (kept: this thread's column) for the norm that scales them.
 template <typename T>
 __device__ __forceinline__ void reinit_jac_node(const T *__restrict__ ps, const uint8_t fl, Ptr6<const T> d,
                                                 const T lc, T *__restrict__ W, Ptr6<T> mu, const Grid &g, int i,
-                                                int j, int k, long long c)
+                                                int j, int k, long long c, T (*kept)[BX * BY])
 {
     T dist[6];
     const int qmin = reinit_distances(fl, d, c, g, dist);
@@ -346,31 +372,28 @@ __device__ __forceinline__ void reinit_jac_node(const T *__restrict__ ps, const 
     const T dtv = T(0.3) * dmin;
     const bool neg = fl & CLS_MASK;
     const T sgn = neg ? T(-1) : T(1);
+    const int tid = threadIdx.y * BX + threadIdx.x;
 
-    // pass 1: the derivative pairs and the partials of the Godunov norm
     T gq[3], S = T(0);
-    bool back[3];
 #pragma unroll 1
     for (int ax = 0; ax < 3; ++ax) {
-        T p[7], df, db;
+        T p[7], jac[7], gs;
         adj_line7(ps, g, i, j, k, c, ax, p);
-        weno5_pair_values<T>(p, (T)axis_h(g, ax), df, db);
-        S = add_rn(S, godunov_axis(neg, df, db, gq[ax], back[ax]));
+        S = add_rn(S, reinit_axis(p, (T)axis_h(g, ax), neg, gs, jac));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) gq[a] = a == ax ? gs : gq[a];
+#pragma unroll
+        for (int o = 0; o < 7; ++o) kept[ax * 7 + o][tid] = jac[o];
     }
     const T G = sqrt(S);
     const T dG = G > T(0) ? T(0.5) / G : T(0);  // zero derivative of sqrt at 0
     const T s_dt = dtv * sgn;
-
-    // pass 2: per axis, partials of the side taken, scaled into the slots
     T *w = W + c;
-#pragma unroll 1
-    for (int ax = 0; ax < 3; ++ax) {
-        T p[7], jac[7], D;
-        adj_line7(ps, g, i, j, k, c, ax, p);
-        const T gs = gq[ax] * dG * s_dt;
-        weno5_side_grad<T>(p, (T)axis_h(g, ax), back[ax], D, jac);
 #pragma unroll
-        for (int o = 0; o < 7; ++o, w += g.num) *w = lc * (gs * jac[o]);
+    for (int ax = 0; ax < 3; ++ax) {
+        const T gs = gq[ax] * dG * s_dt;
+#pragma unroll
+        for (int o = 0; o < 7; ++o, w += g.num) *w = lc * (gs * kept[ax * 7 + o][tid]);
     }
     // d step / d dist_q: through dt for the minimum
     if (fl & (1u << qmin)) mu.p[qmin][c] -= lc * ((G - T(1)) * sgn * T(0.3));
@@ -390,7 +413,9 @@ __device__ __forceinline__ void adj_append(bool pred, unsigned value, unsigned *
 }
 
 // dense pass: fixed nodes get zero slots; nodes with a sign change next to them on any
-// axis are listed for k_adj_reinit_jac_band; the rest are done here
+// axis are listed for k_adj_reinit_jac_band; the rest are done here.  Bound by its instructions
+// (77 % of the issue slots at two passes over the axes): 173 us at 128^3 with general quotients and
+// both sides' partials, 142 on short quotients and one side, 120 with each axis visited once.
 template <typename T>
 __global__ void __launch_bounds__(BX *BY) k_adj_reinit_jac(const T *__restrict__ ps, const uint8_t *__restrict__ flags,
                                                              Ptr6<const T> d, const T *__restrict__ lam, T coef,
@@ -418,7 +443,8 @@ __global__ void __launch_bounds__(BX *BY) k_adj_reinit_jac(const T *__restrict__
         for (int s = 0; s < SLOTS; ++s) W[(long long)s * g.num + c] = T(0);
         return;
     }
-    reinit_jac_node<T>(ps, fl, d, coef * __ldg(lam + c), W, mu, g, i, j, k, c);
+    __shared__ T kept[SLOTS][BX * BY];
+    reinit_jac_node<T>(ps, fl, d, coef * __ldg(lam + c), W, mu, g, i, j, k, c, kept);
 }
 
 // The listed nodes (40,000 around a sphere of radius 38), BAND_NODES at a time, as (node, axis) tasks: the derivative pairs first, then,
@@ -532,7 +558,7 @@ __global__ void __launch_bounds__(BAND_THREADS) k_adj_reinit_jac_band(const T *_
 
 // ---------------------------------------------------------------------------------------
 // transpose pass: out_j = alpha * lam_j - sum of W over the stencil positions equal to j
-// (+ acc_j)
+// (+ acc_j); the share of lam that the step's start takes is added up in the same pass
 // Bound by memory: 185 MB of slots at 128^3, 42 us (4.4 TB/s beside the write-back of the slots);
 // with clamped 64-bit index arithmetic and first pages first it took 54.
 // ---------------------------------------------------------------------------------------
@@ -542,7 +568,7 @@ struct GatherOffsets {
 };
 template <typename T>
 __global__ void __launch_bounds__(BX *BY) k_adj_gather(const T *__restrict__ W, const T *lam, T alpha,
-                                                         const T *__restrict__ acc, T *out, GatherOffsets from, Grid g)
+                                                         const T *acc, T *out, AdjShare<T> share, GatherOffsets from, Grid g)
 {
     // last pages first: theirs are the slots that the pass before wrote last, still in L2
     const int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y, k = gridDim.z - 1 - blockIdx.z;
@@ -561,6 +587,7 @@ __global__ void __launch_bounds__(BX *BY) k_adj_gather(const T *__restrict__ W, 
         }
     }
     const T l = lam[c], a = acc ? acc[c] : T(0);
+    if (share.acc) share.acc[c] = (share.init ? T(0) : share.acc[c]) + (T)share.a * l;
     T s = T(0);
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
@@ -584,14 +611,6 @@ __global__ void __launch_bounds__(BX *BY) k_adj_gather(const T *__restrict__ W, 
         }
     }
     out[c] = alpha * l - s + a;
-}
-
-// acc = (init ? 0 : acc) + a * lam
-template <typename T>
-__global__ void k_adj_axpy(T *acc, const T *__restrict__ lam, T a, bool init, long long n)
-{
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        acc[t] = (init ? T(0) : acc[t]) + a * lam[t];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -706,20 +725,13 @@ cudaError_t launch_adj_reinit_jac(const T *ps, const uint8_t *flags, Ptr6<const 
 }
 
 template <typename T>
-cudaError_t launch_adj_gather(const T *W, const T *lam, double alpha, const T *acc, T *out, const Grid &g,
-                              cudaStream_t s)
+cudaError_t launch_adj_gather(const T *W, const T *lam, double alpha, const T *acc, T *out, AdjShare<T> share,
+                              const Grid &g, cudaStream_t s)
 {
     const long long stride[3] = {g.rows, 1, g.plane};
     GatherOffsets from;
     for (int q = 0; q < SLOTS; ++q) from.at[q] = q * g.num - (q % 7 - 3) * stride[q / 7];
-    k_adj_gather<T><<<node_grid(g), dim3(BX, BY), 0, s>>>(W, lam, (T)alpha, acc, out, from, g);
-    return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch_adj_axpy(T *acc, const T *lam, double a, bool init, const Grid &g, cudaStream_t s)
-{
-    k_adj_axpy<T><<<adj_list_blocks(), 256, 0, s>>>(acc, lam, (T)a, init, g.num);
+    k_adj_gather<T><<<node_grid(g), dim3(BX, BY), 0, s>>>(W, lam, (T)alpha, acc, out, share, from, g);
     return cudaGetLastError();
 }
 
@@ -737,9 +749,8 @@ cudaError_t launch_adj_dist_edges(const T *f, EdgeLists e, Ptr6<const T> mu, T *
                                                   Ptr3<T>, const Grid &, cudaStream_t);                             \
     template cudaError_t launch_adj_reinit_jac<T>(const T *, const uint8_t *, Ptr6<const T>, const T *, double, T *, \
                                                   Ptr6<T>, NodeList, const Grid &, cudaStream_t);                   \
-    template cudaError_t launch_adj_gather<T>(const T *, const T *, double, const T *, T *, const Grid &,            \
-                                              cudaStream_t);                                                        \
-    template cudaError_t launch_adj_axpy<T>(T *, const T *, double, bool, const Grid &, cudaStream_t);              \
+    template cudaError_t launch_adj_gather<T>(const T *, const T *, double, const T *, T *, AdjShare<T>,           \
+                                              const Grid &, cudaStream_t);                                          \
     template cudaError_t launch_adj_dist_edges<T>(const T *, EdgeLists, Ptr6<const T>, T *, const Grid &,          \
                                                   cudaStream_t);
 

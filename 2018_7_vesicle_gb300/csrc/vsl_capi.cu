@@ -1610,15 +1610,13 @@ int rk3_reverse(const T *s0, const T *s1, const T *s2, T *lam, AdjWork<T> &w, co
 {
     // stage 2: out = 1/3 s0 + 2/3 (s2 - step(s2))
     VSL_TRY(jac(s2, lam, 2.0 / 3.0));
-    VSL_TRY(launch_adj_axpy<T>(w.acc, lam, 1.0 / 3.0, true, g, s));
-    VSL_TRY(launch_adj_gather<T>(w.W, lam, 2.0 / 3.0, nullptr, w.x, g, s));
+    VSL_TRY(launch_adj_gather<T>(w.W, lam, 2.0 / 3.0, nullptr, w.x, AdjShare<T>{w.acc, 1.0 / 3.0, true}, g, s));
     // stage 1: s2 = 3/4 s0 + 1/4 (s1 - step(s1))
     VSL_TRY(jac(s1, w.x, 0.25));
-    VSL_TRY(launch_adj_axpy<T>(w.acc, w.x, 0.75, false, g, s));
-    VSL_TRY(launch_adj_gather<T>(w.W, w.x, 0.25, nullptr, w.x, g, s));
+    VSL_TRY(launch_adj_gather<T>(w.W, w.x, 0.25, nullptr, w.x, AdjShare<T>{w.acc, 0.75, false}, g, s));
     // stage 0: s1 = s0 - step(s0)
     VSL_TRY(jac(s0, w.x, 1.0));
-    VSL_TRY(launch_adj_gather<T>(w.W, w.x, 1.0, w.acc, lam, g, s));
+    VSL_TRY(launch_adj_gather<T>(w.W, w.x, 1.0, w.acc, lam, AdjShare<T>{}, g, s));
     return VSL_OK;
 }
 
@@ -1705,7 +1703,7 @@ int op_reinit_adjoint(const T *F0, int iteration, T *lam, T *tape, int rows, int
     }
     // the distances' dependence on F0
     VSL_TRY(launch_adj_dist_edges<T>(F0, re.edges, cview(w.mu), w.W, g, s));
-    VSL_TRY(launch_adj_gather<T>(w.W, lam, 1.0, nullptr, lam, g, s));
+    VSL_TRY(launch_adj_gather<T>(w.W, lam, 1.0, nullptr, lam, AdjShare<T>{}, g, s));
     return VSL_OK;
 }
 

@@ -268,11 +268,15 @@ cudaError_t launch_adj_advect_jac(const T *ps, Ptr3<const T> v, const double *dt
 template <typename T>
 cudaError_t launch_adj_reinit_jac(const T *ps, const uint8_t *flags, Ptr6<const T> d, const T *lam, double coef, T *W,
                                   Ptr6<T> mu, NodeList band, const Grid &g, cudaStream_t s);
+// a stage's adjoint also passes `a` of lam on to the step's start: acc = (init ? 0 : acc) + a lam
+template <typename T> struct AdjShare {
+    T *acc = nullptr;
+    double a = 0.0;
+    bool init = false;
+};
 template <typename T>
-cudaError_t launch_adj_gather(const T *W, const T *lam, double alpha, const T *acc, T *out, const Grid &g,
-                              cudaStream_t s);
-template <typename T>
-cudaError_t launch_adj_axpy(T *acc, const T *lam, double a, bool init, const Grid &g, cudaStream_t s);
+cudaError_t launch_adj_gather(const T *W, const T *lam, double alpha, const T *acc, T *out, AdjShare<T> share,
+                              const Grid &g, cudaStream_t s);
 template <typename T>
 cudaError_t launch_adj_dist_edges(const T *f, EdgeLists e, Ptr6<const T> mu, T *W, const Grid &g, cudaStream_t s);
 constexpr int ADJ_SLOTS = 21;
