@@ -18,9 +18,9 @@
 //     nonuniform stencils for a few of its lanes; the WENO kinds run them as tasks sorted by
 //     stencil kind (vsl_band.cuh), on the same short quotients.
 //   * scaled differences are formed once per tile and shared through shared memory.
-// About 280 / 320 FP64 instructions per node and stage (transport / norm), the pipe 85% busy.  Per
-// stage at 128^3 on GB300: advection 1.13 ms, extension 1.23 ms, reinitialization 1.43 ms (3.2,
-// 3.7 and 3.7 ms one node per thread with general quotients).
+// 288 / 370 FP64 instructions per node and stage (transport / norm, band included; ncu), the pipe
+// 86% busy.  Per stage at 128^3 on GB300: advection 1.13 ms, extension 1.17 ms, reinitialization
+// 1.40 ms (3.2, 3.7 and 3.7 ms one node per thread with general quotients).
 //
 // The sequences above need operands away from overflow and underflow.  A node whose stencil
 // holds a value that is neither zero nor of magnitude 2^-400 .. 2^100 (infinities and NaN
