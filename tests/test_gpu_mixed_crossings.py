@@ -93,3 +93,14 @@ def test_extension_against_fp64(size, eno3):
         out.append(f(sdf3.as_field(C.float(), t), 5).double())
     err = float((out[0] - out[1]).norm() / out[1].norm())
     assert err <= 5e-5, err
+
+
+@pytest.mark.parametrize("size", [(31, 7, 3), (33, 17, 40), (70, 64, 61), (160, 150, 140)])
+def test_area_and_volume_terms_over_the_block(size):
+    """The FP32 form's FP64 terms of the promoted field, pooled per warp and per block, against the
+    plain form on that field: the same terms to a few FP64 roundings each, summed in another order."""
+    grid = grid_of(size)
+    F = field_of(grid, size, "smooth")
+    a32, a64 = (sdf3.SDF3(grid, Val=F.to(t), precision=p).area_volume().cpu().numpy()
+                for t, p in ((torch.float32, "f32"), (torch.float64, "f64")))
+    assert np.all(np.abs(a32 - a64) <= 1e-11 * np.abs(a64)), (a32, a64)
