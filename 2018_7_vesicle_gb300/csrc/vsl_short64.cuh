@@ -20,7 +20,10 @@ namespace {
 __device__ __forceinline__ double quotient(double a, double d, double r)
 {
     const double q = __dmul_rn(a, r);
-    return __fma_rn(__fma_rn(-d, q, a), r, q);
+    const double z = __fma_rn(__fma_rn(-d, q, a), r, q);
+    // the first product's sign: the correction would turn a quotient of -0 into +0
+    return __hiloint2double((__double2hiint(z) & 0x7fffffff) | (__double2hiint(q) & (int)0x80000000),
+                            __double2loint(z));
 }
 
 // 1 / d to within an ulp for a normal d whose reciprocal is normal

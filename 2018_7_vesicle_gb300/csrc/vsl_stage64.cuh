@@ -1,5 +1,6 @@
 // vsl_stage64.cuh -- stage kernels of the plain FP64 form on cheaper arithmetic with the
-// same results, bit for bit, as the per-node functions of vsl_fused.cuh.
+// same results as the per-node functions of vsl_fused.cuh: bit for bit but for the sign of a zero
+// (a transport stage adds no zero of the side it does not evaluate).
 //
 // What bounds these kernels is the FP64 pipe: two lanes per SM and clock on GB300, 1/64 of
 // the FP32 rate, so a warp's FP64 instruction occupies it for 16 cycles and everything else
