@@ -2,21 +2,23 @@
 //
 // The FP64 pipe bounds those kernels (two lanes per SM and clock on GB300), and a general
 // division is about ten of its instructions.  A quotient whose divisor's reciprocal is known
-// takes three: multiply, remainder, correction (Markstein, IBM J. Res. Dev. 34, 1990), and is
-// the correctly rounded one.  A reciprocal takes three more, from the documented PTX
-// approximation rcp.approx.ftz.f64 (20 bits) and one third-order Newton step (its error is that
-// of the approximation cubed), and serves every quotient by the same divisor.  Neither handles
-// overflow or underflow: the callers check their operands' range and keep the general code for
-// the rest.  (tests/test_quotient_host.py replays both on the CPU.)
+// takes three: multiply, remainder, correction.  With the correctly rounded reciprocal it is the
+// correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990; Brisebarre, Muller and Raina,
+// IEEE Trans. Comput. 53, 2004).  A reciprocal takes three more and serves every quotient by the
+// same divisor.  Neither handles overflow or underflow (nor an intermediate that underflows): the
+// callers check their operands' range and keep the general code for the rest.
+// (tests/test_quotient_exact_host.py runs this file on the CPU.)
 #pragma once
 
 #include <cmath>
 #include <cuda_runtime.h>
 
+#include "vsl_device.cuh"
+
 namespace vsl {
 namespace {
 
-// a / d for the divisor d whose reciprocal r is 1 / d to within an ulp
+// a / d for the divisor d whose reciprocal is r
 __device__ __forceinline__ double quotient(double a, double d, double r)
 {
     const double q = __dmul_rn(a, r);
@@ -26,13 +28,25 @@ __device__ __forceinline__ double quotient(double a, double d, double r)
                             __double2loint(z));
 }
 
-// 1 / d to within an ulp for a normal d whose reciprocal is normal
+// 1 / d for a normal d whose reciprocal is normal, as the quotients above need it: with a
+// reciprocal y off the exact one by (1/2 + e) ulp a quotient can round wrongly only if the
+// divisor's significand (in 1 .. 2) is at least 2 - 4 e.  The hardware's FP32 reciprocal of the
+// significand is within 2^-22.4 and one third-order Newton step cubes that, so e is 2^-15; divisors
+// next to two (the upper 2^-12) take one more step, which rounds correctly (Markstein) but for the
+// significand of ones alone, whose reciprocal is the odd one next to a power of two.  The seed is
+// integer work and free beside the FP64 pipe.
 __device__ __forceinline__ double reciprocal(double d)
 {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = __fma_rn(-d, y, 1.0);  // at most about 2^-19
-    return __fma_rn(y, __fma_rn(e, e, e), y);
+    const int hi = __double2hiint(d), lo = __double2loint(d);
+    const int s = __float_as_int(rcp_ftz(__int_as_float(0x3f800000 | ((hi << 3 | (int)((unsigned)lo >> 29)) & 0x7fffff))));
+    double y = __hiloint2double(((s >> 3) + ((896 + 1023) << 20) - (hi & 0x7ff00000)) | (hi & (int)0x80000000), s << 29);
+    const double e = __fma_rn(-d, y, 1.0);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    if (__builtin_expect((hi & 0xfff00) == 0xfff00, 0)) {
+        y = __fma_rn(y, __fma_rn(-d, y, 1.0), y);
+        if ((hi & 0xfffff) == 0xfffff && lo == -1) y = __hiloint2double(__double2hiint(y), __double2loint(y) | 1);
+    }
+    return y;
 }
 
 // magnitude bits of the high word
