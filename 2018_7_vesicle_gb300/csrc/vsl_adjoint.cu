@@ -80,10 +80,12 @@ __device__ __forceinline__ void adj_line7(const T *__restrict__ f, const Grid &g
 
 // Number types of the uniform stencils: quotients as a shared reciprocal, a product and a
 // remainder correction (vsl_short64.cuh), three to six instructions where a general quotient is
-// about twenty; a node took 38 of them per axis.  FP32: the hardware reciprocal is within an ulp,
-// and a Newton step from there gives the correctly rounded one, the quotient then too (Markstein's
-// theorems), so the values are those of general quotients.  Both need operands away from overflow
-// and underflow (uniform_range); other nodes take the general quotients.
+// about twenty; a node took 38 of them per axis.  FP32: a Newton step from the hardware reciprocal
+// gives the correctly rounded one for every significand (an ulp's error would do but for the
+// significand of ones; sm_103a has that one right, tests/test_gpu_quotient32.py), and the quotient
+// is then the correctly rounded one (Markstein's theorems), +0 for -0.  Operands near overflow take
+// the general quotients (uniform_range).  In FP64 those near underflow do as well; in FP32 a
+// numerator below about 2^-100, whose remainder is no normal number, leaves an ulp's error.
 struct Short32 {
     float v;
     __device__ __forceinline__ Short32() {}

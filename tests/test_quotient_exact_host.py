@@ -126,3 +126,82 @@ def test_short_quotients_are_correctly_rounded(lib, seed_ulp):
     assert lib.edges(seed_ulp) == 0
     assert lib.midpoints(400_000, seed_ulp) == 0
     assert lib.random_pairs(500_000, seed_ulp) == 0
+
+
+# The FP32 quotient of the adjoint's uniform stencils (Short32 of csrc/vsl_adjoint.cu): the hardware
+# reciprocal is either neighbour of the exact one, and the correctly rounded one for the significand
+# of ones (tests/test_gpu_quotient32.py).
+SHIM32 = r"""
+static float __fmul_rn(float a, float b) { volatile float r = a * b; return r; }
+static float __fmaf_rn(float a, float b, float c) { return std::fmaf(a, b, c); }
+static float neighbour(float x)
+{
+    const double exact = 1.0 / (double)x;
+    const float y = (float)exact;
+    if ((~cast<uint32_t>(x) & 0x7fffff) == 0) return y;
+    if (seed_ulp < 0) return (double)y > exact ? std::nextafterf(y, 0.f) : y;
+    return (double)y < exact ? std::nextafterf(y, INFINITY) : y;
+}
+#define rcp_ftz neighbour
+"""
+CHECK32 = r"""
+static uint32_t s32 = 2463534242u;
+static uint32_t rnd32() { s32 ^= s32 << 13; s32 ^= s32 >> 17; s32 ^= s32 << 5; return s32; }
+static float sig32(uint32_t m, int e) { return std::ldexp((float)((m & 0x7fffff) | 0x800000), e - 23); }
+static bool wrong32(float a, float b)
+{
+    volatile float want = a / b;
+    return (Short32(a) / Short32(b)).v != want;
+}
+/* every divisor's significand against powers of two and their neighbours, a weight of the scheme, a
+   random numerator and those whose quotients lie nearest to the midpoint of two neighbours */
+extern "C" long all_significands(int ulp)
+{
+    seed_ulp = ulp;
+    long bad = 0;
+    const uint32_t one = 1u << 23;
+    for (uint32_t m = 0; m < one; ++m) {
+        const float b = sig32(m, (int)(m % 41) - 20);
+        bad += wrong32(1.f, b) + wrong32(-0x1.fffffep3f, b) + wrong32(0.6f, b) + wrong32(sig32(rnd32(), 0), b);
+        const uint64_t D = m | one;
+        if (D % 2 == 0) continue;
+        uint64_t inv = D;
+        for (int it = 0; it < 6; ++it) inv *= 2 - D * inv;
+        for (int k = 24; k <= 25; ++k)
+            for (int sign = -1; sign <= 1; sign += 2) {
+                const uint64_t M = (sign > 0 ? inv : 0 - inv) & ((1ULL << k) - 1);
+                const uint64_t A = (D * M - (uint64_t)(int64_t)sign) >> k;
+                if (M >= 2 * one && M < 4 * one && A >= one && A < 2 * one) bad += wrong32((float)A, (float)D);
+            }
+    }
+    return bad;
+}
+/* numerators down to 2^-100 over divisors of 1 .. 2 */
+extern "C" long small_numerators(long n, int ulp)
+{
+    seed_ulp = ulp;
+    long bad = 0;
+    for (long q = 0; q < n; ++q) bad += wrong32(sig32(rnd32(), -(int)(rnd32() % 101)), sig32(rnd32(), 0));
+    return bad;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib32(tmp_path_factory):
+    with open(os.path.join(CSRC, "vsl_adjoint.cu")) as f:
+        struct = re.search(r"^struct Short32 \{.*?^\};", f.read(), flags=re.M | re.S).group(0)
+    d = tmp_path_factory.mktemp("quotient32")
+    (d / "q.cpp").write_text(SHIM + SHIM32 + struct + CHECK32)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-o", str(d / "q.so"),
+                    str(d / "q.cpp")], check=True)
+    so = ctypes.CDLL(str(d / "q.so"))
+    so.all_significands.restype, so.all_significands.argtypes = ctypes.c_long, [ctypes.c_int]
+    so.small_numerators.restype, so.small_numerators.argtypes = ctypes.c_long, [ctypes.c_long, ctypes.c_int]
+    return so
+
+
+@pytest.mark.parametrize("seed_ulp", [-1, 1])
+def test_fp32_short_quotients_are_correctly_rounded(lib32, seed_ulp):
+    assert lib32.all_significands(seed_ulp) == 0
+    assert lib32.small_numerators(1_000_000, seed_ulp) == 0
