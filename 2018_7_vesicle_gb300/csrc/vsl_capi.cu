@@ -63,8 +63,8 @@ template <typename T> struct ReinitWork {
     uint8_t *flags;
     Ptr6<T> dist;     // ENO3 only
     EdgeLists edges;  // ENO3 only (its setDistance)
-    Band band;         // FP32 form
-    NodeList flagged;  // FP64 form: nodes with a distance flag
+    Band band;                           // FP32 form
+    NodeList flagged{nullptr, nullptr};  // FP64 form: nodes with a distance flag
 };
 template <typename T> ReinitWork<T> carve_reinit(Bump &w, const Grid &g, bool own_dist)
 {
@@ -75,7 +75,17 @@ template <typename T> ReinitWork<T> carve_reinit(Bump &w, const Grid &g, bool ow
     for (int q = 0; q < 6; ++q) r.dist.p[q] = own_dist ? w.take<T>(g.num) : nullptr;
     r.edges = own_dist ? carve_edges(w, g) : EdgeLists{};
     r.band = carve_band<T>(w, g);
-    r.flagged = std::is_same<T, double>::value ? carve_list(w, g) : NodeList{nullptr, nullptr};
+    // FP64: the flagged nodes take the edges' storage, which is free once the distances are set
+    if (own_dist && std::is_same<T, double>::value && r.b)
+        r.flagged = NodeList{r.edges.idx[0], r.edges.count + 3};
+    return r;
+}
+
+// the same with caller's distances: the FP64 form's list has no storage to share
+template <typename T> ReinitWork<T> carve_reinit_listed(Bump &w, const Grid &g)
+{
+    ReinitWork<T> r = carve_reinit<T>(w, g, false);
+    if (std::is_same<T, double>::value) r.flagged = carve_list(w, g);
     return r;
 }
 
@@ -121,7 +131,7 @@ template <typename T> struct TolWork {
 template <typename T> TolWork<T> carve_tol(Bump &w, const Grid &g)
 {
     TolWork<T> t;
-    t.re = carve_reinit<T>(w, g, false);
+    t.re = carve_reinit_listed<T>(w, g);
     t.max_bits = w.take<unsigned long long>(2);  // the ticket shares the second word
     t.ticket = t.max_bits ? reinterpret_cast<unsigned *>(t.max_bits + 1) : nullptr;
     return t;
@@ -262,7 +272,7 @@ size_t measure(int op, const Grid &g, int elem)
     auto run = [&](auto tag) {
         using T = decltype(tag);
         switch (op) {
-        case VSL_OP_REINIT_WENO5: carve_reinit<T>(w, g, false); break;
+        case VSL_OP_REINIT_WENO5: carve_reinit_listed<T>(w, g); break;
         case VSL_OP_REINIT_ENO3: carve_reinit<T>(w, g, true); break;
         case VSL_OP_EXTEND_WENO5: carve_extend<T>(w, g, false); break;
         case VSL_OP_EXTEND_ENO3: carve_extend<T>(w, g, true); break;
@@ -504,7 +514,7 @@ int op_reinit_weno5(T *F, int iteration, const T *xpr, const T *xpl, const T *yp
     Grid g = make_grid(rows, cols, pges, dx, dy, dz);
     if (int st = check_ws(VSL_OP_REINIT_WENO5, g, sizeof(T), ws, bytes)) return st;
     Bump b(ws);
-    ReinitWork<T> w = carve_reinit<T>(b, g, false);
+    ReinitWork<T> w = carve_reinit_listed<T>(b, g);
     Ptr6<const T> d = six(xpr, xpl, ypf, ypb, zpu, zpd);
     VSL_TRY(launch_classify<T>(F, d, w.flags, w.flagged, g, s));
     return reinit_loop<T>(F, iteration, d, w, g, false, s);
@@ -1591,6 +1601,7 @@ int op_relax_step(T *F, T *xpr, T *xpl, T *ypf, T *ypb, T *zpu, T *zpd, double A
     VSL_TRY(launch_sum_partials(w.red.partials, nb, 1, ds3, ene, s));
     if (reinit_iters > 0) {
         const Ptr6<const T> d = six<T>(xpr, xpl, ypf, ypb, zpu, zpd);
+        if (std::is_same<T, double>::value) w.re.flagged = w.ext.flagged;  // the extensions are done
         VSL_TRY(launch_classify<T>(F, d, w.re.flags, w.re.flagged, g, s));
         return reinit_loop<T>(F, reinit_iters, d, w.re, g, false, s);
     }
@@ -1701,7 +1712,8 @@ int op_reinit_adjoint(const T *F0, int iteration, T *lam, T *tape, int rows, int
         if (int st = reinit_stages<T>(phik, d, re, g, s)) return st;
         if (int st = rk3_reverse<T>(phik, re.b, re.c, lam, w, g, s, jac)) return st;
     }
-    // the distances' dependence on F0
+    // the distances' dependence on F0 (the FP64 form's list of flagged nodes took the edges' storage)
+    if (std::is_same<T, double>::value) VSL_TRY(launch_set_distance<T>(F0, re.dist, g, true, re.edges, s));
     VSL_TRY(launch_adj_dist_edges<T>(F0, re.edges, cview(w.mu), w.W, g, s));
     VSL_TRY(launch_adj_gather<T>(w.W, lam, 1.0, nullptr, lam, AdjShare<T>{}, g, s));
     return VSL_OK;
