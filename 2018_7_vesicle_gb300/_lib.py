@@ -40,6 +40,7 @@ SIGNATURES = {
     # tuning table of the tiled kernels (pages per block)
     "vsl_set_tile_pages": "iiiii",
     "vsl_tile_pages": "iiii",
+    "vsl_launch_pages": "iiii",
     # plane loads of the tiled kernels (1 TMA, 0 registers) and the TMA wait-timeout count
     "vsl_set_plane_loads": "i",
     "vsl_plane_loads": "",

@@ -5,8 +5,10 @@ pages mean more blocks and more parallelism on small grids, more pages mean fewe
 reloads per node on large ones.  The library keeps a table of pages per (grid shape,
 stage kind) (vsl_set_tile_pages / vsl_tile_pages of the C ABI); `tune_shape` fills it for
 one level-set object by timing each kind's own operation (extension, reinitialization,
-advection, ENORK2 extension and reinitialization) on that object's field for every candidate, with CUDA events, and keeping
-the fastest.  Tune before recording CUDA graphs: a graph keeps the launch shapes it was
+advection, ENORK2 extension and reinitialization) on that object's field for every candidate,
+with CUDA events, and keeping the fastest.  Among the candidates is the page count that the
+library takes by itself for the shape (`launch_pages`), unless the caller lists the
+candidates.  Tune before recording CUDA graphs: a graph keeps the launch shapes it was
 recorded with.
 """
 from __future__ import annotations
@@ -17,7 +19,7 @@ from ._lib import lib
 from .sdf3 import SDF3, colmajor_full
 
 KINDS = {"reinit": 0, "extend": 1, "advect": 2, "enork2_extend": 3, "enork2_reinit": 4}
-CANDIDATES = (4, 8, 10, 15, 16, 20, 25, 30, 32, 40, 64)
+CANDIDATES = (1, 2, 3, 4, 8, 10, 15, 16, 20, 25, 30, 32, 40, 64)
 DEFAULT_PAGES = 20  # most pages per block of a shape not in the table (small grids: fewer)
 # tile of one block of the tiled kernels, fixed at compile time: 32x4, 32x16 and 64x4 tiles
 # gave bitwise the same results and ran -1 % / +4 % / +1 % on the 256^3 vesicle step and
@@ -47,6 +49,12 @@ def wave_candidates(size, sms: int | None = None, fill: float = 0.85, max_waves:
 
 def get_pages(size, kind: str) -> int:
     return int(lib().raw("vsl_tile_pages", *size, KINDS[kind]))
+
+
+def launch_pages(size, kind: str) -> int:
+    """Pages per block that an operation on a single grid of this shape launches with on the
+    current device: the table's, or the library's own choice (a batch: `get_pages`)."""
+    return int(lib().raw("vsl_launch_pages", *size, KINDS[kind]))
 
 
 def set_pages(size, kind: str, pages: int) -> None:
@@ -105,10 +113,12 @@ def tune_shape(sdf: SDF3, candidates=CANDIDATES, iters: int = 2, reps: int = 3, 
     """Pick pages per block for each stage kind on sdf's grid shape; returns
     {kind: {"pages": best, "ms": {candidate: time}}}.  sdf must be FP32 with its
     distances set (setDistance).  candidates="waves" takes wave_candidates(shape); `kinds`
-    limits the tuning to those stage kinds (all of KINDS by default)."""
+    limits the tuning to those stage kinds (all of KINDS by default).  The untuned launch is
+    one of the candidates (launch_pages) unless they are given as a list of the caller's."""
     if sdf.precision != "f32":
         raise ValueError("the tiled kernels are the FP32 form's")
     size = sdf.GD3.Size
+    own = isinstance(candidates, str) or candidates is CANDIDATES
     if isinstance(candidates, str):
         if candidates != "waves":
             raise ValueError("candidates: a sequence of page counts or 'waves'")
@@ -127,7 +137,9 @@ def tune_shape(sdf: SDF3, candidates=CANDIDATES, iters: int = 2, reps: int = 3, 
         if kinds is not None and kind not in kinds:
             continue
         times = {}
-        for c in _candidates(size[2], candidates):
+        set_pages(size, kind, 0)
+        untuned = [launch_pages(size, kind)] if own else []
+        for c in untuned + [c for c in _candidates(size[2], candidates) if c not in untuned]:
             set_pages(size, kind, c)
             times[c] = _elapsed_ms(fn, reps)
         best = min(times, key=times.get)

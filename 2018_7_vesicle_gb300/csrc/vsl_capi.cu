@@ -1798,6 +1798,12 @@ int vsl_tile_pages(int rows, int cols, int pges, int kind)
     return tile_pages(make_grid(rows, cols, pges, 1.0, 1.0, 1.0), kind);
 }
 
+int vsl_launch_pages(int rows, int cols, int pges, int kind)
+{
+    if (rows <= 0 || cols <= 0 || pges <= 0 || kind < 0 || kind > 4) return 0;
+    return launch_pages(make_grid(rows, cols, pges, 1.0, 1.0, 1.0), kind);
+}
+
 size_t vsl_workspace_bytes(int op, int rows, int cols, int pges, int elem_bytes)
 {
     if (rows <= 0 || cols <= 0 || pges <= 0) return 0;

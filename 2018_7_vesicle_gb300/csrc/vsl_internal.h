@@ -212,6 +212,7 @@ cudaError_t launch_shadow_init(const float *c, double *shadow, NodeList list, cu
 // pages per block of the tiled kernels for a grid shape and kind (the tuning table, or the
 // default); set_tile_pages(..., 0) restores the default
 int tile_pages(const Grid &g, int kind);
+int launch_pages(const Grid &g, int kind);  // of a single grid's launch on the current device
 int set_tile_pages(int rows, int cols, int pges, int kind, int pages);
 
 // ---- toolbox and reductions (vsl_toolbox.cu) ------------------------------------------

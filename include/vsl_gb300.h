@@ -196,11 +196,14 @@ enum {
  * ENORK2 reinitialization, used by every later launch of that shape (a CUDA graph keeps the
  * value it was recorded with).
  * Shapes not in the table use 20, and fewer where a single grid would not fill the GPU with
- * that many (the batch entry points keep 20).  vsl_set_tile_pages(..., pages = 0) removes an entry; it returns
- * VSL_ERR_SHAPE / VSL_ERR_VALUE for a bad shape, kind or pages (1..65535), or a full
- * table (512 entries).  vsl_tile_pages returns the table's value or 20 (0 for bad input). */
+ * that many (the batch entry points keep 20).  vsl_set_tile_pages(..., pages = 0) removes an
+ * entry; it returns VSL_ERR_SHAPE / VSL_ERR_VALUE for a bad shape, kind or pages (1..65535),
+ * or a full table (512 entries).  vsl_tile_pages returns the table's value or 20, which the
+ * batch entry points launch with, vsl_launch_pages the value that the operations on a single
+ * grid launch with on the current device (0 for bad input, both). */
 int vsl_set_tile_pages(int rows, int cols, int pges, int kind, int pages);
 int vsl_tile_pages(int rows, int cols, int pges, int kind);
+int vsl_launch_pages(int rows, int cols, int pges, int kind);
 
 /* Plane loads of the FP32 tiled stage kernels (no counterpart in the reference), process-wide:
  * mode 0 (the default) loads every plane through registers; mode 1 loads them by TMA tensor
