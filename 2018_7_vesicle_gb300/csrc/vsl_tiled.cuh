@@ -991,41 +991,49 @@ int tile_pages(const Grid &g, int kind)
     return set ? set : VSL_TILED_KZ;
 }
 
-
-// Pages per block of a single-grid launch: the tuning table's, else the one of PAGES that the
-// cost below puts lowest.  A block marches its pages at a rate that the blocks resident on its
-// SM share once `share` of them do (fewer leave issue slots idle), and loads planes worth about
-// 1.5 pages before its first one; the busiest SM holds ceil(blocks / SMs) of them.  The page
-// loop is unrolled by five, so counts above five are multiples of it.  The extension keeps the
-// default where its band is not run as tasks: its time is then its band blocks' chain, whatever
-// the pages.  Measured on GB300, us per stage, 20 pages / this rule /
-// the best of 1 .. 32: reinitialization 64^3 27.2 / 14.2 / 14.2, 96^3 32.1 / 22.1 / 22.1, 128^3
-// 44.6 / 37.0 / 37.0; ENORK2 extension 64^3 11.0 / 4.7 / 4.7, 96^3 11.5 / 8.8 / 8.1, 128^3 16.8 /
-// 14.4 / 14.2; advection 64^3 11.4 / 5.1 / 5.1, 128^3 21.2 / 21.2 / 20.5; WENO5
-// extension (tasks) 64^3 11.5 / 7.7 / 7.5, 96^3 15.9 / 14.4 / 13.5.  From about 192^3 on
-// the rule is the default.  (A batch's grids share one launch and keep the default.)
+// Pages per block of a single-grid launch: the tuning table's, else the default or the one of PAGES
+// that the cost below puts lowest, and at least 5 % below the default's.  A block marches its
+// pages (no more than the grid has) at a rate that the blocks resident on its SM share once `share`
+// of them do (fewer leave issue slots idle), and loads planes worth about 1.5 pages before its
+// first one; the busiest SM holds ceil(blocks / SMs) of them.  The extensions' band blocks run
+// beside the tile blocks only while those are at most `room` to an SM; behind them they add their
+// chain.  The WENO5 extension's band takes as long as eight pages, so shorter blocks gain nothing,
+// and it keeps the default where its band is not run as tasks (its time is then the chain,
+// whatever the pages).  The page loop is unrolled by five, so counts above five are multiples of
+// it.  Measured on GB300, us per stage, 20 pages / this rule / the best of 1 .. 20:
+// reinitialization 64^3 27.2 / 14.2 / 14.2, 96^3 32.1 / 22.1 / 22.1, 128^3 44.6 / 37.0 / 37.0; ENORK2
+// extension 64^3 11.0 / 4.7 / 4.7, 96^3 11.5 / 8.8 / 8.1, 128^3 16.8 / 14.4 / 14.2, 300 x 300 x 6 the
+// default (4 pages: +19 %); advection 64^3 11.4 / 5.1 / 5.1, 128^3 21.2 / 21.2 / 20.5; WENO5
+// extension 64^3 11.5 / 7.7 / 7.5, 96^3 ten pages, 7 % below the default (five: 2 % above), 300 x 300
+// x 6 the default (5 pages: +31 %).  Over 22 shapes from 24^3 to 1500 x 1200 x 1 with two bands each
+// no kind is slower than at 20 pages by more than 1.5 %.  From about 192^3 on the rule is the default.  (A batch's grids share
+// one launch and keep the default.)
 int launch_pages(const Grid &g, int kind)
 {
     if (const int set = tile_pages_set(g, kind)) return set;
     if (kind == SK_EXTEND && g.num > EXTEND_TASKS_GRID) return VSL_TILED_KZ;
-    static constexpr int PAGES[] = {1, 2, 3, 4, 5, 10, VSL_TILED_KZ};
-    int share = 4, least = 1;
-    if (kind == SK_EXTEND) share = 3, least = 5;
+    static constexpr int PAGES[] = {10, 5, 4, 3, 2, 1};
+    constexpr double CHAIN = 15.0;
+    int share = 4, least = 1, shortest = 0;
+    double room = 0.0;
+    if (kind == SK_EXTEND) share = 3, least = 5, shortest = 8, room = 2.6;
     if (kind == SK_ADVECT || kind == SK_VELOCITY) share = 2;
-    if (kind == SK_ENO2) share = 5, least = 4;
+    if (kind == SK_ENO2) share = 5, least = 4, room = 4.4;
     if (kind == SK_ENO2R) least = 2;
     const long long sms = list_blocks() / 4;
     const long long tiles = (long long)((g.rows + TY - 1) / TY) * ((g.cols + TX - 1) / TX);
-    int best = VSL_TILED_KZ;
-    double lowest = 0.0;
-    for (int p : PAGES) {
-        if (p < least) continue;
+    auto cost = [&](int p) {
         const long long blocks = tiles * ((g.pges + p - 1) / p);
-        const double cost = (p + 1.5) * (double)std::max<long long>(share, (blocks + sms - 1) / sms);
-        if (lowest == 0.0 || cost <= lowest) {
-            lowest = cost;
-            best = p;
-        }
+        const double march = (std::max(std::min(p, g.pges), shortest) + 1.5) *
+                             (double)std::max<long long>(share, (blocks + sms - 1) / sms);
+        return room > 0.0 && (double)blocks > room * (double)sms ? march + CHAIN : march;
+    };
+    int best = VSL_TILED_KZ;
+    double lowest = 0.95 * cost(VSL_TILED_KZ);
+    for (int p : PAGES) {
+        if (p < least || cost(p) >= lowest) continue;
+        lowest = cost(p);
+        best = p;
     }
     return best;
 }
