@@ -16,6 +16,9 @@
 // node per thread: 30 WENO5 extension pseudo-steps 32^3 0.84 / 1.27, 64^3 1.03 / 1.41, 96^3
 // 1.61 / 1.78, 128^3 2.86 / 2.85, 192^3 7.16 / 6.92; 30 reinitialization pseudo-steps 32^3
 // 1.35 / 1.48, 64^3 1.56 / 1.73, 128^3 3.92 / 3.98; a stage of 160^3 68.0 / 65.3 us.
+// So do dense bands (folded or many interfaces) on small grids: ten reinitialization pseudo-steps of
+// 64^3 with 35,000 / 53,000 / 191,000 band nodes 0.715 / 0.725, 0.812 / 0.744, 1.43 / 1.05, of 128^3
+// with 32,000 / 126,000 / 1,530,000 1.41 / 1.42, 2.03 / 1.79, 9.2 / 6.0 (10 shapes, 9 bands each).
 #pragma once
 
 #include <cstdint>
@@ -27,9 +30,9 @@ namespace {
 
 enum BandTask { BT_FORE = 0, BT_BACK = 1, BT_UNIFORM = 2, BT_KINDS = 3 };
 // the largest grids (nodes) whose reinitialization and extension bands run as tasks in the mixed
-// form, and the most band nodes of an extension that do
+// form, and the most band nodes that do
 constexpr long long REINIT_TASKS_GRID = 128LL * 128 * 128, EXTEND_TASKS_GRID = 112LL * 112 * 112;
-constexpr unsigned EXTEND_TASKS_MOST = 20000;
+constexpr unsigned EXTEND_TASKS_MOST = 20000, REINIT_TASKS_MOST = 40000;
 
 // the shared memory of a chunk of N nodes
 template <typename T, int N> struct BandChunk {

@@ -794,11 +794,8 @@ __global__ void __launch_bounds__(TY *TX, (KIND == SK_ENO2 ? 5 : VSL_TILED_MIN_B
 // stage's counter for its next use.  (The static bands of the other kinds run in band
 // blocks of the tiled launch itself, k_stage_tiled.)  No occupancy target (75 registers;
 // 8 blocks per SM gained nothing).
-template <bool ENO3>
-__global__ void __launch_bounds__(128) k_band_stage(TiledArgs a, unsigned *next_counter)
+template <bool ENO3> __device__ __forceinline__ void reinit_band_nodes(const TiledArgs &a, unsigned n)
 {
-    const unsigned n = *a.counter;
-    if (next_counter && blockIdx.x == 0 && threadIdx.x == 0) *next_counter = 0u;
     const Grid &g = a.g;
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const long long c = a.queue[t];
@@ -809,13 +806,26 @@ __global__ void __launch_bounds__(128) k_band_stage(TiledArgs a, unsigned *next_
         reinit_node<float, ENO3, true>(a.phi_s, a.phi_n, a.out, a.flags, a.d, g, a.stage, i, j, k);
     }
 }
-// the same band as sorted tasks (vsl_band.cuh), on grids of up to REINIT_TASKS_GRID nodes
+template <bool ENO3>
+__global__ void __launch_bounds__(128) k_band_stage(TiledArgs a, unsigned *next_counter)
+{
+    const unsigned n = *a.counter;
+    if (next_counter && blockIdx.x == 0 && threadIdx.x == 0) *next_counter = 0u;
+    reinit_band_nodes<ENO3>(a, n);
+}
+// the same band as sorted tasks (vsl_band.cuh) up to REINIT_TASKS_MOST nodes, on grids of up to
+// REINIT_TASKS_GRID nodes
 template <bool ENO3>
 __global__ void __launch_bounds__(128) k_band_tasks(const __grid_constant__ TiledArgs a, unsigned *next_counter)
 {
+    const unsigned n = *a.counter;
     if (next_counter && blockIdx.x == 0 && threadIdx.x == 0) *next_counter = 0u;
+    if (n > REINIT_TASKS_MOST) {
+        reinit_band_nodes<ENO3>(a, n);
+        return;
+    }
     __shared__ typename ReinitBand<ENO3>::Chunk ch;
-    run_band<128>(ReinitBand<ENO3>{a}, ch, *a.counter, blockIdx.x, gridDim.x, threadIdx.x);
+    run_band<128>(ReinitBand<ENO3>{a}, ch, n, blockIdx.x, gridDim.x, threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------------------
