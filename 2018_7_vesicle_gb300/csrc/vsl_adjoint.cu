@@ -267,12 +267,13 @@ __device__ __noinline__ void iface_side_jac(const T p[7], T h, T r1, T l1, bool 
 // Bound by its instructions (about 1000 per node, 60 % of the issue slots) and the 176 MB of slots
 // that it writes at 128^3 (30 % of the memory rate).  The next axis' line and velocity adjoint are
 // loaded while an axis is formed, and the slots' addresses advance by additions: 105 -> 93 us.
+// FP32: five blocks to an SM; FP64, bound by its pipe, two (no spills; forward and adjoint of four
+// steps at 96^3 30.3 ms, 30.5 at five blocks and 48 registers, with four or three between).
 // ---------------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(BX *BY, 5) k_adj_advect_jac(const T *__restrict__ ps, Ptr3<const T> v,
-                                                             const double *__restrict__ dt,
-                                                             const T *__restrict__ lam, T coef, T *__restrict__ W,
-                                                             Ptr3<T> gv, Grid g)
+__global__ void __launch_bounds__(BX *BY, (sizeof(T) == 4 ? 5 : 2))
+    k_adj_advect_jac(const T *__restrict__ ps, Ptr3<const T> v, const double *__restrict__ dt,
+                     const T *__restrict__ lam, T coef, T *__restrict__ W, Ptr3<T> gv, Grid g)
 {
     int i, j, k;
     long long c;
