@@ -1,7 +1,8 @@
 // vsl_tool64.cuh -- one node of the plain FP64 calculus toolbox (set_calculus_toolbox.cu:9-107),
 // the reference's expressions in its order, on a number type R: double, or Short64 (the same
 // roundings on the short quotients of vsl_short64.cuh) where the node's values are ordinary.
-// Included by files compiled without multiply-add contraction.
+// The kernels that take it are in files compiled without multiply-add contraction (vsl_toolbox.cu,
+// vsl_plain.cu); vsl_auxi.cuh takes the divisors and the range test in both precisions.
 //
 // What bounds it is the FP64 pipe: with general divisions and every field formed at every node a
 // node took about 560 FP64 instructions.  Here a field is formed only where it is wanted.
