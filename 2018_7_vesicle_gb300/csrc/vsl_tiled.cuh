@@ -596,10 +596,15 @@ struct ExtendBand {
         extension_differences(a, sh, c, L, ax, r1 < h, l1 < h, cs, p, pv, dd);
 #pragma unroll
         for (int m = 0; m < 6; ++m) dd[m] = dd[m] / G[m];
+        auto side = [&](bool back) {
+            return a.eno3 ? nonuniform_side_dd<float, true>(G, dd, back) : nonuniform_side_dd<float, false>(G, dd, back);
+        };
         const bool back = kind == BT_BACK;
-        const float D = a.eno3 ? nonuniform_side_dd<float, true>(G, dd, back)
-                               : nonuniform_side_dd<float, false>(G, dd, back);
-        (back ? ch.db : ch.df)[ax][node] = D;
+        (back ? ch.db : ch.df)[ax][node] = side(back);
+        // the other side is multiplied by zero, which leaves it out only where it is finite: not where
+        // the values are not, or the weights may overflow (NaN fails the comparison)
+        const float sum = fabsf(dd[0]) + fabsf(dd[1]) + fabsf(dd[2]) + fabsf(dd[3]) + fabsf(dd[4]) + fabsf(dd[5]);
+        if (!(sum < 1e4f)) (back ? ch.df : ch.db)[ax][node] = side(!back);
     }
     __device__ __forceinline__ void finish(const Chunk &ch, int node) const
     {
