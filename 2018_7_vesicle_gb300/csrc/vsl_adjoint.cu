@@ -103,11 +103,23 @@ struct Short32 {
         return __fmaf_rn(__fmaf_rn(-b.v, q, a.v), y, q);
     }
 };
+// FP64: as Short64, with sums and products that the compiler may fuse as it does in the general
+// code of this file
+struct Fused64 {
+    double v;
+    __device__ __forceinline__ Fused64() {}
+    __device__ __forceinline__ Fused64(double x) : v(x) {}
+    __device__ __forceinline__ Fused64(int x) : v((double)x) {}
+    friend __device__ __forceinline__ Fused64 operator+(Fused64 a, Fused64 b) { return a.v + b.v; }
+    friend __device__ __forceinline__ Fused64 operator-(Fused64 a, Fused64 b) { return a.v - b.v; }
+    friend __device__ __forceinline__ Fused64 operator*(Fused64 a, Fused64 b) { return a.v * b.v; }
+    friend __device__ __forceinline__ Fused64 operator/(Fused64 a, Fused64 b) { return quotient(a.v, b.v, reciprocal(b.v)); }
+};
 __device__ __forceinline__ float adj_raw(Short32 x) { return x.v; }
-__device__ __forceinline__ double adj_raw(Short64 x) { return x.v; }
+__device__ __forceinline__ double adj_raw(Fused64 x) { return x.v; }
 __device__ __forceinline__ float adj_raw(float x) { return x; }
 __device__ __forceinline__ double adj_raw(double x) { return x; }
-template <typename T> using ShortOf = typename std::conditional<std::is_same<T, float>::value, Short32, Short64>::type;
+template <typename T> using ShortOf = typename std::conditional<std::is_same<T, float>::value, Short32, Fused64>::type;
 
 // do the scaled differences of a line allow the short quotients (NaN fails the comparison)
 __device__ __forceinline__ float max3_nan(float a, float b, float c)
