@@ -146,34 +146,37 @@ __global__ void __launch_bounds__(NT) k_toolbox64(const double *__restrict__ f, 
     }
 }
 
-// result[q] = scale * sum_b partials[ncomp*b + q], ncomp <= 4, in a fixed order (one block of 1024):
-// per thread, per warp by shuffles, then the warps.  One block has one SM's FP64 pipe, 16 cycles a
-// warp's instruction, and that and the chain of additions are its time: warps past the last
-// partial are left out (their sums are exact zeros), and the components go side by side, each
-// summed over the warps by a thread of its own (48^3, 432 partials of 2: 7.3 -> 4.3 us).
-__global__ void __launch_bounds__(1024) k_sum_partials(const double *__restrict__ partials, int nblocks, int ncomp,
-                                                       double scale, double *__restrict__ result)
+// result[q] = scale * sum_b partials[NC*b + q] in a fixed order (one block of 1024): per thread, per
+// warp by shuffles, then the warps.  One block has one SM's FP64 pipe, 16 cycles a warp's
+// instruction, and that and the chain of additions are its time: warps past the last partial are
+// left out (their sums are exact zeros), and the components go side by side, each summed over the
+// warps by a thread of its own (48^3, 432 partials of 2: 7.3 -> 4.3 us).  With many partials it
+// waits on their loads, eight rows of which are in flight (the component count is the compiler's,
+// so that no branch parts them: SUMLINE).
+template <int NC>
+__global__ void __launch_bounds__(1024) k_sum_partials(const double *__restrict__ partials, int nblocks, double scale,
+                                                       double *__restrict__ result)
 {
-    __shared__ double s[4][32];
+    __shared__ double s[NC][32];
     const int warp = threadIdx.x >> 5, warps = min((int)(blockDim.x >> 5), (nblocks + 31) >> 5);
     if (warp < warps) {
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        // unrolled so that the loads are in flight together; the additions keep their order
-#pragma unroll 4
+        double acc[NC];
+#pragma unroll
+        for (int q = 0; q < NC; ++q) acc[q] = 0.0;
+        // the additions keep their order
+#pragma unroll 8
         for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (q < ncomp) acc[q] += partials[(long long)ncomp * b + q];
+            for (int q = 0; q < NC; ++q) acc[q] += partials[(long long)NC * b + q];
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (q >= ncomp) break;
+        for (int q = 0; q < NC; ++q) {
             acc[q] = warp_sum(acc[q]);
             if ((threadIdx.x & 31) == 0) s[q][warp] = acc[q];
         }
     }
     __syncthreads();
-    if ((int)threadIdx.x < ncomp) {
+    if (threadIdx.x < NC) {
         double tot = 0.0;
         for (int w = 0; w < warps; ++w) tot += s[threadIdx.x][w];
         result[threadIdx.x] = tot * scale;
@@ -209,7 +212,12 @@ int toolbox_partial_blocks(const Grid &g)
 cudaError_t launch_sum_partials(const double *partials, int nblocks, int ncomp, double scale, double *result,
                                 cudaStream_t s)
 {
-    k_sum_partials<<<1, 1024, 0, s>>>(partials, nblocks, ncomp, scale, result);
+    switch (ncomp) {
+    case 1: k_sum_partials<1><<<1, 1024, 0, s>>>(partials, nblocks, scale, result); break;
+    case 2: k_sum_partials<2><<<1, 1024, 0, s>>>(partials, nblocks, scale, result); break;
+    case 4: k_sum_partials<4><<<1, 1024, 0, s>>>(partials, nblocks, scale, result); break;
+    default: return cudaErrorInvalidValue;
+    }
     return cudaGetLastError();
 }
 
