@@ -799,24 +799,37 @@ __global__ void __launch_bounds__(TY *TX, (KIND == SK_ENO2 ? 5 : VSL_TILED_MIN_B
 // stage's counter for its next use.  (The static bands of the other kinds run in band
 // blocks of the tiled launch itself, k_stage_tiled.)  No occupancy target (75 registers;
 // 8 blocks per SM gained nothing).
-template <bool ENO3> __device__ __forceinline__ void reinit_band_nodes(const TiledArgs &a, unsigned n)
+template <bool ENO3>
+__device__ __forceinline__ void reinit_band_nodes(const unsigned *__restrict__ queue, unsigned n,
+                                                  const float *__restrict__ phi_s, const float *__restrict__ phi_n,
+                                                  float *__restrict__ out, const uint8_t *__restrict__ flags,
+                                                  const Ptr6<const float> &d, const Grid &g, int stage)
 {
-    const Grid &g = a.g;
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const long long c = a.queue[t];
+        const long long c = queue[t];
         const int k = (int)(c / g.plane);
         const long long r = c - (long long)k * g.plane;
         const int j = (int)(r / g.rows);
         const int i = (int)(r - (long long)j * g.rows);
-        reinit_node<float, ENO3, true>(a.phi_s, a.phi_n, a.out, a.flags, a.d, g, a.stage, i, j, k);
+        reinit_node<float, ENO3, true>(phi_s, phi_n, out, flags, d, g, stage, i, j, k);
     }
+}
+// out of line, on its own arguments: inlined beside the tasks the compiler fused other products of
+// the node's code
+template <bool ENO3>
+__device__ __noinline__ void reinit_band_call(const unsigned *__restrict__ queue, unsigned n,
+                                              const float *__restrict__ phi_s, const float *__restrict__ phi_n,
+                                              float *__restrict__ out, const uint8_t *__restrict__ flags,
+                                              Ptr6<const float> d, Grid g, int stage)
+{
+    reinit_band_nodes<ENO3>(queue, n, phi_s, phi_n, out, flags, d, g, stage);
 }
 template <bool ENO3>
 __global__ void __launch_bounds__(128) k_band_stage(TiledArgs a, unsigned *next_counter)
 {
     const unsigned n = *a.counter;
     if (next_counter && blockIdx.x == 0 && threadIdx.x == 0) *next_counter = 0u;
-    reinit_band_nodes<ENO3>(a, n);
+    reinit_band_nodes<ENO3>(a.queue, n, a.phi_s, a.phi_n, a.out, a.flags, a.d, a.g, a.stage);
 }
 // the same band as sorted tasks (vsl_band.cuh) up to REINIT_TASKS_MOST nodes, on grids of up to
 // REINIT_TASKS_GRID nodes
@@ -826,7 +839,7 @@ __global__ void __launch_bounds__(128) k_band_tasks(const __grid_constant__ Tile
     const unsigned n = *a.counter;
     if (next_counter && blockIdx.x == 0 && threadIdx.x == 0) *next_counter = 0u;
     if (n > REINIT_TASKS_MOST) {
-        reinit_band_nodes<ENO3>(a, n);
+        reinit_band_call<ENO3>(a.queue, n, a.phi_s, a.phi_n, a.out, a.flags, a.d, a.g, a.stage);
         return;
     }
     __shared__ typename ReinitBand<ENO3>::Chunk ch;

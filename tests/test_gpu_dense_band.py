@@ -31,3 +31,21 @@ def test_dense_band_is_the_batched_form(pkg, vsl, period, dense):
     A = torch.sin(3 * x) * torch.cos(2 * y) + 0.5 * z**2 + F
     got = m.WENORK3ClosetPointSurfaceRedistance(A, 2, 1)
     assert torch.equal(got, B.redistance_batched([m], [A], 2, 1, eno3=True)[0])
+
+
+@pytest.mark.parametrize("eno3", [False, True])
+def test_redistance_of_a_wavy_field(pkg, vsl, eno3):
+    """A surface field with 78,000 band nodes on an odd box, redistanced: the reinitialization stages
+    see the extensions' outputs, whose values reach more of the stencils' branches."""
+    B = importlib.import_module(pkg.__name__ + ".batch")
+    S = importlib.import_module(pkg.__name__ + ".shapes")
+    rows, cols, pges = 161, 113, 97
+    half = [1.5 * n / rows if n < rows else 1.5 for n in (cols, rows, pges)]
+    v = [np.linspace(-max(1.15, b), max(1.15, b), n) for b, n in zip(half, (cols, rows, pges))]
+    x, y, z = S.meshgrid(*v, device="cuda")
+    F = torch.sqrt(x**2 / 0.8 + y**2 / 0.6 + z**2 / 0.5) - 0.9 + 0.02 * torch.sin(2 * x + y - 1.5 * z)
+    A = torch.sin(3 * x + 0.8) * torch.cos(2 * y + 0.2) + 0.5 * z**2
+    m = pkg.SDF3(pkg.GD3(x, y, z, spacing=tuple(float(a[1] - a[0]) for a in v)), Val=F, precision="f32")
+    fn = m.WENORK3ClosetPointSurfaceRedistance if eno3 else m.WENO5RK3ClosetPointSurfaceRedistance
+    for it, ext in ((1, 1), (3, 2)):
+        assert torch.equal(fn(A, it, ext), B.redistance_batched([m], [A], it, ext, eno3=eno3)[0])
