@@ -462,7 +462,8 @@ __global__ void __launch_bounds__(BX *BY) k_adj_reinit_jac(const T *__restrict__
     reinit_jac_node<T>(ps, fl, d, coef * __ldg(lam + c), W, mu, g, i, j, k, c, kept);
 }
 
-// The listed nodes (40,000 around a sphere of radius 38), BAND_NODES at a time, as (node, axis) tasks: the derivative pairs first, then,
+// The listed nodes (40,000 around a sphere of radius 38), BAND_NODES at a time, as (node, axis)
+// tasks: the derivative pairs first, then,
 // once the norm of each node is known, the partials, with the tasks in order of kind (uniform,
 // interface-aware forward, interface-aware backward) so that a warp takes one path.  Bound by
 // fetching the instructions of the dual-number code, eight warps to a multiprocessor (255

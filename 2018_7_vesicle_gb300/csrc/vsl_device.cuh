@@ -502,8 +502,9 @@ __device__ __noinline__ void weno_nonuniform_pair(const T xs[7], const T hs[7], 
     d_back = nu_combine(v, c, s);
 }
 
-// One side of weno_nonuniform_pair alone, from the divided differences dd[m] = (hs[m+1] - hs[m]) / (xs[m+1] - xs[m]); the forward one does not
-// read dd[0], the backward one not dd[5].
+// One side of weno_nonuniform_pair alone, from the divided differences
+// dd[m] = (hs[m+1] - hs[m]) / (xs[m+1] - xs[m]); the forward one does not read dd[0], the backward
+// one not dd[5].
 template <typename T> __device__ __forceinline__ T weno_nonuniform_fore(const T xs[7], const T dd[6])
 {
     T e[6], u[5], v[3], c[3], s[3];

@@ -34,7 +34,8 @@ __device__ __forceinline__ double quotient(double a, double d, double r)
 // significand is within 2^-22.4 and one third-order Newton step cubes that, so e is 2^-15; divisors
 // next to two (the upper 2^-12) take one more step, which rounds correctly (Markstein) but for the
 // significand of ones alone, whose reciprocal is the odd one next to a power of two.  The seed is
-// integer work and free beside the FP64 pipe.
+// integer work and free beside the FP64 pipe (against a seed of 20 bits and no guard: steps of 128^3
+// and up 0.5 .. 1.2 % faster, 64^3 reinitializations, which wait on the chain, 1.4 % slower).
 __device__ __forceinline__ double reciprocal(double d)
 {
     const int hi = __double2hiint(d), lo = __double2loint(d);

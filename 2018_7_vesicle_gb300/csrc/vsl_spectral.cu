@@ -189,7 +189,8 @@ int launch_smooth_bilaplacian(const T *rhs, T *out, const double *dt, double alp
         if (r != CUFFT_SUCCESS) return VSL_ERR_CUDA;
         const int parts = g.rows + g.cols + g.pges;
         if (parts <= FILTER_TABLE)
-            k_spectral_filter<T, true><<<spec_blocks() / 8, FILTER_THREADS, parts * sizeof(double), s>>>(spec, g, dt, alpha, exact ? 1 : 0);
+            k_spectral_filter<T, true><<<spec_blocks() / 8, FILTER_THREADS, parts * sizeof(double), s>>>(spec, g, dt, alpha,
+                                                                                                   exact ? 1 : 0);
         else
             k_spectral_filter<T, false><<<spec_blocks() / 8, FILTER_THREADS, 0, s>>>(spec, g, dt, alpha, exact ? 1 : 0);
         if (cudaGetLastError() != cudaSuccess) return VSL_ERR_CUDA;

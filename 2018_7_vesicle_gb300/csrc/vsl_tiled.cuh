@@ -33,9 +33,10 @@ namespace {
 
 // Pages per block (a launch parameter: the default below, or the value the tuning table
 // holds for the grid shape and stage kind) and the occupancy target (compile time).
-// The default is measured on GB300 at 256^3 (smaller grids: launch_pages), vesicle step as a graph: 4 blocks per SM (64 registers) beat
-// 5 (48 registers with spills) at 16/32/64 pages; with the page loop unrolled by the ring
-// length, 10/15/16/20/25/30/32/40 pages gave 33.6/33.0/33.1/32.7/32.4/32.8/33.0/32.9 ms.
+// The default is measured on GB300 at 256^3 (smaller grids: launch_pages), vesicle step as a
+// graph: 4 blocks per SM (64 registers) beat 5 (48 registers with spills) at 16/32/64 pages; with
+// the page loop unrolled by the ring length, 10/15/16/20/25/30/32/40 pages gave
+// 33.6/33.0/33.1/32.7/32.4/32.8/33.0/32.9 ms.
 #ifndef VSL_TILED_KZ
 #define VSL_TILED_KZ 20
 #endif
